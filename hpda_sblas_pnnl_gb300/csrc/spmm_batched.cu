@@ -312,6 +312,7 @@ int sblas_batch_plan_create(int nmat, const sblas_batch_matrix *mats, int k, int
     a.head_val = reinterpret_cast<double *>(base + b_mats + 4 * b_int);
     a.tail_val = reinterpret_cast<double *>(base + b_mats + 4 * b_int + b_val);
     a.nunits = nunits;
+    a.unit_nnz = (int)unit;
     a.override_xy = 0;
     e = cudaMemcpyAsync(base, dm.data(), sizeof(Mat) * nmat, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) {

@@ -41,8 +41,7 @@
 #include <climits>
 #include <mutex>
 
-#include <utility>
-
+#include "launch.cuh"
 #include "ptx.cuh"
 #include "sblas_internal.h"
 
@@ -1011,26 +1010,6 @@ int configure_shape(int *out_bps, size_t *out_smem)
     *out_bps = bps;
     if (out_smem) *out_smem = smem_request[dev];
     return SBLAS_OK;
-}
-
-// A launch with programmatic stream serialisation: the kernel may start
-// while the previous kernel of the stream finishes, and waits for it
-// (ptx::griddep_wait) before it reads global memory.
-template <class... KArgs, class... Args>
-cudaError_t launch_pdl(void (*kfn)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                       cudaStream_t stream, Args &&...args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kfn, std::forward<Args>(args)...);
 }
 
 template <int SIGMA, int VK, int AB, class Src = TileArgs>

@@ -1,0 +1,57 @@
+"""Sizes at which a kernel or a rule that chooses one can go wrong: run
+lengths, tile remainders, the smallest and largest sizes of a path.  The
+checker is the oracle; bars as in the other GPU tests (relative L2 <= 1e-12
+for FP64 sums in another order, whole numbers equal)."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+RTOL_L2 = 1e-12
+
+
+def rel_l2(y, ref):
+    den = np.linalg.norm(ref)
+    num = np.linalg.norm(np.asarray(y) - ref)
+    return num / den if den > 0 else num
+
+
+def csr_of_lengths(lengths, n, seed, cuda):
+    """A CSR matrix with the given row lengths, random columns and values."""
+    rng = np.random.default_rng(seed)
+    rowptr = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
+    col = rng.integers(0, n, rowptr[-1]).astype(np.int32)
+    val = rng.standard_normal(rowptr[-1])
+    return (rowptr, col, val), tuple(torch.from_numpy(a).to(cuda) for a in (rowptr, col, val))
+
+
+@pytest.mark.parametrize("k", [1, 2, 4, 8, 16])
+def test_batch_fixup_run_lengths(sblas_lib, cuda, k):
+    """Rows over 1, 31, 32, 33 units, over the last run a warp takes and the
+    first the whole block takes, and the longest, side by side."""
+    from hpda_sblas_pnnl_gb300 import ops
+    s, unit, wg = 4, 128, 32 // k
+    edge = 64 * wg * unit
+    lengths = [5, 1, 3 * unit, 0, 31 * unit, 32 * unit - 3, 33 * unit, 7, edge - unit, edge + unit,
+               0, 0, 2 * edge + 17, 40 * unit, 2, 33 * unit, 33 * unit + 1, 1]
+    n = 5000
+    (rp, col, val), dev = csr_of_lengths(lengths, n, 11 + k, cuda)
+    m = len(lengths)
+    g = torch.Generator(device=cuda)
+    g.manual_seed(k)
+    shape = (lambda r: (r, k) if k > 1 else (r,))
+    x = torch.randn(shape(n), generator=g, dtype=torch.float64, device=cuda)
+    y0 = torch.randn(shape(m), generator=g, dtype=torch.float64, device=cuda)
+    plan = ops.SpmmPlan(*dev, n=n, k=k, s=s)
+    y = y0.clone()
+    plan(x, y, 1.5, -0.5)
+    first = y.clone()
+    ref = O.csr_spmm(m, n, rp, col, val, x.cpu().numpy().reshape(n, k),
+                     y0.cpu().numpy().reshape(m, k), 1.5, -0.5)
+    assert rel_l2(y.cpu().numpy().reshape(m, k), ref) <= RTOL_L2
+    y.copy_(y0)
+    plan(x, y, 1.5, -0.5)
+    assert torch.equal(y, first)      # the same bits on every run
