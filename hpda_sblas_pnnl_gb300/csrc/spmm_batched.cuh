@@ -1035,6 +1035,16 @@ cudaError_t shape_grid(int nunits, int *grid)
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kfn, CTA, smem)) != cudaSuccess)
         return e;
+    // The lanes-over-columns shapes past 196 KB of shared memory per SM (S = 16
+    // and 32 with FP64 values) run one CTA fewer in the 196-KB carveout, not
+    // all in the 228-KB one with 28 KB of L1: the lines of X and of permuted
+    // values live there.  1M rows, 20.0M nonzeros, K = 16, S = 16: product 657
+    // -> 653 us, transposed product 1046 -> 792 us; K = 8: 398 -> 390, 910 -> 577.
+    if (use_vec<K>() && (size_t)bps * (smem + 1024) > 196 * 1024) {
+        e = cudaFuncSetAttribute(kfn, cudaFuncAttributePreferredSharedMemoryCarveout, 85);
+        if (e != cudaSuccess) return e;
+        bps = (int)(196 * 1024 / (smem + 1024));
+    }
     if (bps < 1) return cudaErrorInvalidConfiguration;
     const long long need = (nunits + NW - 1) / NW;
     const long long full = (long long)sms * bps;
@@ -1050,7 +1060,7 @@ namespace sblas {
 namespace batch {
 
 // Compiled shapes: K in {1, 2, 4, 8, 16} (one translation unit each),
-// S in {4, 8, 16, 32}, every value kind.  Op::GRID computes the persistent
+// S in {4, 8, 16, 32} (and 1, 2 for K >= 8), every value kind.  Op::GRID computes the persistent
 // grid of the shape into *grid_out; SPMM and SDDMM launch.
 template <int K, int S, int VK>
 cudaError_t launch_sddmm(const Args &a, int grid, cudaStream_t stream)
@@ -1077,6 +1087,10 @@ cudaError_t dispatch_k(Op op, int S, int VK, const Args *a, int nunits, int grid
                                  : shape_grid<K, SS, VV>(nunits, grid_out);
 #define SBLAS_BATCH_S(SS)                                                                \
     SBLAS_BATCH_SHAPE(SS, VAL_F64) SBLAS_BATCH_SHAPE(SS, VAL_F32) SBLAS_BATCH_SHAPE(SS, VAL_PATTERN)
+    if constexpr (use_vec<K>()) {   // chosen by the plan for small matrices only
+        SBLAS_BATCH_S(1)
+        SBLAS_BATCH_S(2)
+    }
     SBLAS_BATCH_S(4)
     SBLAS_BATCH_S(8)
     SBLAS_BATCH_S(16)

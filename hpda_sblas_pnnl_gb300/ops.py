@@ -326,7 +326,7 @@ class BatchPlan:
     descriptors to the device and partitions all matrices into units of
     32*s nonzeros; each call is one persistent kernel plus the carry fix-up
     (sblas_batch_spmm): no allocation, no copy, graph-capturable.  s = 0
-    takes the library default for k (see tune.batch_s for a measured pick).
+    lets the library pick by k and size (see tune.batch_s for a measured pick).
     """
 
     def __init__(self, matrices, xs, ys, k: int, alpha: float = 1.0, beta: float = 0.0,

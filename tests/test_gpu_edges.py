@@ -55,3 +55,26 @@ def test_batch_fixup_run_lengths(sblas_lib, cuda, k):
     y.copy_(y0)
     plan(x, y, 1.5, -0.5)
     assert torch.equal(y, first)      # the same bits on every run
+
+
+@pytest.mark.parametrize("k", [1, 2, 4, 8, 16])
+@pytest.mark.parametrize("nnz", [3_000, 20_000, 250_000, 500_000, 1_300_000, 2_100_000])
+def test_plan_picks_a_shape_for_every_size(sblas_lib, cuda, k, nnz):
+    """s = 0 on both sides of each size at which the pick changes, with a
+    permuted transpose product: forward and both gradients."""
+    from hpda_sblas_pnnl_gb300 import autograd
+    rng = np.random.default_rng(nnz + k)
+    m = max(50, nnz // 20)
+    lengths = rng.multinomial(nnz, rng.dirichlet(np.ones(m)))
+    (rp, col, val), (trp, tcol, tval) = csr_of_lengths(lengths, m, nnz + k, cuda)
+    op = autograd.CsrOperator(trp, tcol, m, k)
+    x = torch.from_numpy(rng.standard_normal((m, k))).to(cuda)
+    gy = torch.from_numpy(rng.standard_normal((m, k))).to(cuda)
+    y = op.forward(tval, x)
+    ref = O.csr_spmm(m, m, rp, col, val, x.cpu().numpy(), np.zeros((m, k)))
+    assert rel_l2(y.cpu().numpy(), ref) <= RTOL_L2
+    dx = op.grad_x(tval, gy)
+    assert rel_l2(dx.cpu().numpy(), O.csr_spmm_t(m, m, rp, col, val, gy.cpu().numpy())) <= RTOL_L2
+    dval = op.grad_val(gy, x)
+    assert rel_l2(dval.cpu().numpy(), O.csr_sddmm(m, m, rp, col, gy.cpu().numpy(),
+                                                   x.cpu().numpy())) <= RTOL_L2
