@@ -399,6 +399,43 @@ int sblas_csr_filter_x(int m, long long nnz, const int *rowptr, const int *col,
                                work_bytes, static_cast<cudaStream_t>(stream));
 }
 
+int sblas_dspmspv(int kernel, int m, int n, long long nnz, double alpha, const double *val,
+                  const int *rowptr, const int *col, const double *x, double beta, double *y,
+                  void *work, size_t work_bytes, void *stream)
+{
+    clear_error();
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (m < 0 || n < 0 || nnz < 0 || nnz >= 0x7fffffffLL) {
+        set_error(SBLAS_ERR_ARG, "bad sizes m=%d n=%d nnz=%lld", m, n, nnz);
+        return SBLAS_ERR_ARG;
+    }
+    if (kernel < 1 || kernel > 3) {
+        set_error(SBLAS_ERR_ARG, "kernel must be 1, 2 or 3 (got %d)", kernel);
+        return SBLAS_ERR_ARG;
+    }
+    if (m == 0) return SBLAS_OK;
+    if (y == nullptr || (nnz > 0 && (rowptr == nullptr || col == nullptr || x == nullptr))) {
+        set_error(SBLAS_ERR_ARG, "null device pointer");
+        return SBLAS_ERR_ARG;
+    }
+    if (kernel == 1) {
+        if (val == nullptr) {
+            set_error(SBLAS_ERR_UNSUPPORTED, "kernel 1 takes FP64 values only");
+            return SBLAS_ERR_UNSUPPORTED;
+        }
+        return launch_rowsplit_spmv(m, n, nnz, alpha, val, rowptr, col, x, beta, y, st, true);
+    }
+    const int sigma = default_sigma_for(m, nnz);
+    const size_t need = tile_workspace_bytes(nnz, sigma);
+    if (nnz > 0 && (work == nullptr || work_bytes < need ||
+                    (reinterpret_cast<uintptr_t>(work) & 255) != 0)) {
+        set_error(SBLAS_ERR_ARG, "workspace needs %zu bytes at 256-byte alignment", need);
+        return SBLAS_ERR_ARG;
+    }
+    return launch_tile_spmv(m, n, nnz, alpha, val, val ? VAL_F64 : VAL_PATTERN, rowptr, col, x,
+                            beta, y, sigma, work, st, false, true, true);
+}
+
 int sblas_zero(void *p, size_t bytes, void *stream)
 {
     clear_error();

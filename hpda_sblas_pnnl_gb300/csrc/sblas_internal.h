@@ -52,12 +52,14 @@ enum ValueKind { VAL_F64 = 0, VAL_F32 = 1, VAL_PATTERN = 2 };
 // `work` must hold tile_workspace_bytes(nnz, sigma) bytes, 256-byte aligned.
 // analysed = true: the partition of `work` was computed by
 // launch_tile_analyse for this row pointer and sigma (skipped here).
+// skip_zero_x: nonzeros whose x entry is zero are left out (spMspV), and col
+// and val may be longer than rowptr[m]; sigma 11, FP64 or pattern-only.
 // reset_status = false keeps the workspace's status word as it is (a call
 // made of several launches on one workspace clears it once, at its start).
 int launch_tile_spmv(int m, int n, long long nnz, double alpha, const void *val,
                      int val_kind, const int *rowptr, const int *col, const double *x,
                      double beta, double *y, int sigma, void *work, cudaStream_t stream,
-                     bool analysed = false, bool reset_status = true);
+                     bool analysed = false, bool reset_status = true, bool skip_zero_x = false);
 // Status word of a tile workspace (0 = every wait completed), read with a
 // synchronous copy: the caller has synchronised the launches' stream.
 int tile_workspace_status(void *work, int *out);
@@ -101,7 +103,7 @@ int launch_tile_analyse(int m, long long nnz, const int *rowptr, int sigma, void
 // Row-split kernel (one sub-warp per row; kernel version 1).
 int launch_rowsplit_spmv(int m, int n, long long nnz, double alpha, const double *val,
                          const int *rowptr, const int *col, const double *x, double beta,
-                         double *y, cudaStream_t stream);
+                         double *y, cudaStream_t stream, bool skip_zero_x = false);
 
 // y[i] = beta * y[i] (beta == 0 writes exact zeros), for m == 0 / nnz == 0.
 int launch_scale_y(int m, double beta, double *y, cudaStream_t stream);

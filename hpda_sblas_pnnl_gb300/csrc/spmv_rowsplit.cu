@@ -12,7 +12,7 @@
 namespace sblas {
 namespace {
 
-template <int G, int AB>
+template <int G, int AB, bool SKIP>
 __global__ void __launch_bounds__(256) rowsplit_kernel(int m, double alpha, double beta,
                                                        const double *__restrict__ val,
                                                        const int *__restrict__ rowptr,
@@ -27,7 +27,10 @@ __global__ void __launch_bounds__(256) rowsplit_kernel(int m, double alpha, doub
     for (int row = (blockIdx.x * blockDim.x + threadIdx.x) / G; row < m; row += groups) {
         const int b = __ldg(rowptr + row), e = __ldg(rowptr + row + 1);
         double s = 0.0;
-        for (int j = b + lane_g; j < e; j += G) s = fma(__ldg(val + j), __ldg(x + __ldg(col + j)), s);
+        for (int j = b + lane_g; j < e; j += G) {
+            const double xj = __ldg(x + __ldg(col + j));
+            if (!SKIP || xj != 0.0) s = fma(__ldg(val + j), xj, s);
+        }
 #pragma unroll
         for (int o = G / 2; o > 0; o >>= 1) s += __shfl_down_sync(mask, s, o, G);
         if (lane_g == 0) {
@@ -38,7 +41,7 @@ __global__ void __launch_bounds__(256) rowsplit_kernel(int m, double alpha, doub
     }
 }
 
-template <int G>
+template <int G, bool SKIP>
 void launch_g(int m, double alpha, double beta, const double *val, const int *rowptr,
               const int *col, const double *x, double *y, cudaStream_t stream)
 {
@@ -46,28 +49,37 @@ void launch_g(int m, double alpha, double beta, const double *val, const int *ro
     const long long want = ((long long)m * G + threads - 1) / threads;
     const int blocks = (int)(want < 16LL * device_num_sms() ? want : 16LL * device_num_sms());
     if (alpha == 1.0 && beta == 0.0)
-        rowsplit_kernel<G, 0><<<blocks, threads, 0, stream>>>(m, alpha, beta, val, rowptr, col, x, y);
+        rowsplit_kernel<G, 0, SKIP><<<blocks, threads, 0, stream>>>(m, alpha, beta, val, rowptr, col, x, y);
     else if (beta == 0.0)
-        rowsplit_kernel<G, 1><<<blocks, threads, 0, stream>>>(m, alpha, beta, val, rowptr, col, x, y);
+        rowsplit_kernel<G, 1, SKIP><<<blocks, threads, 0, stream>>>(m, alpha, beta, val, rowptr, col, x, y);
     else
-        rowsplit_kernel<G, 2><<<blocks, threads, 0, stream>>>(m, alpha, beta, val, rowptr, col, x, y);
+        rowsplit_kernel<G, 2, SKIP><<<blocks, threads, 0, stream>>>(m, alpha, beta, val, rowptr, col, x, y);
+}
+
+template <bool SKIP>
+void launch_mean(int m, long long nnz, double alpha, const double *val, const int *rowptr,
+                 const int *col, const double *x, double beta, double *y, cudaStream_t stream)
+{
+    const double mean = (double)nnz / (double)m;
+    if (mean <= 2.0) launch_g<2, SKIP>(m, alpha, beta, val, rowptr, col, x, y, stream);
+    else if (mean <= 4.0) launch_g<4, SKIP>(m, alpha, beta, val, rowptr, col, x, y, stream);
+    else if (mean <= 8.0) launch_g<8, SKIP>(m, alpha, beta, val, rowptr, col, x, y, stream);
+    else if (mean <= 16.0) launch_g<16, SKIP>(m, alpha, beta, val, rowptr, col, x, y, stream);
+    else launch_g<32, SKIP>(m, alpha, beta, val, rowptr, col, x, y, stream);
 }
 
 }  // namespace
 
+// skip_zero_x: nonzeros whose x entry is zero are left out
 int launch_rowsplit_spmv(int m, int n, long long nnz, double alpha, const double *val,
                          const int *rowptr, const int *col, const double *x, double beta,
-                         double *y, cudaStream_t stream)
+                         double *y, cudaStream_t stream, bool skip_zero_x)
 {
     (void)n;
     if (m <= 0) return SBLAS_OK;
     if (nnz <= 0) return launch_scale_y(m, beta, y, stream);
-    const double mean = (double)nnz / (double)m;
-    if (mean <= 2.0) launch_g<2>(m, alpha, beta, val, rowptr, col, x, y, stream);
-    else if (mean <= 4.0) launch_g<4>(m, alpha, beta, val, rowptr, col, x, y, stream);
-    else if (mean <= 8.0) launch_g<8>(m, alpha, beta, val, rowptr, col, x, y, stream);
-    else if (mean <= 16.0) launch_g<16>(m, alpha, beta, val, rowptr, col, x, y, stream);
-    else launch_g<32>(m, alpha, beta, val, rowptr, col, x, y, stream);
+    if (skip_zero_x) launch_mean<true>(m, nnz, alpha, val, rowptr, col, x, beta, y, stream);
+    else launch_mean<false>(m, nnz, alpha, val, rowptr, col, x, beta, y, stream);
     SBLAS_CUDA_TRY(cudaGetLastError());
     return SBLAS_OK;
 }

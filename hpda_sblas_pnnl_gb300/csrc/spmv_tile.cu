@@ -326,7 +326,7 @@ __device__ __forceinline__ void produce_tile(const MatView &a, const Smem<SIGMA,
     using L = Layout<SIGMA, VK>;
     using VT = typename ValTraits<VK>::T;
     const long long tb = a.tb;
-    const int cnt = (int)((a.nnz - tb < L::TILE) ? (a.nnz - tb) : L::TILE);
+    const int cnt = (int)max(0ll, (a.nnz - tb < L::TILE) ? (a.nnz - tb) : (long long)L::TILE);
     const int vdone = a.use_tma ? (int)((((long long)cnt * L::VB) & ~15ll) / (L::VB ? L::VB : 1)) : 0;
     const int cdone = a.use_tma ? (int)((((long long)cnt * 4) & ~15ll) / 4) : 0;
     const int nr = R1 - R0;
@@ -409,7 +409,17 @@ __device__ __forceinline__ bool f32_not_normal(unsigned u)
 // buffer of the tile's parity; the chunk's head (first segment of a row
 // begun earlier) and tail (partial of the row crossing the chunk end) are
 // published for the epilogue warp of the tile's parity.  No CTA-wide barrier.
-template <int SIGMA, int VK, int AB, class Src>
+//
+// SKIP (sparse x): a nonzero whose x entry is zero contributes nothing, also
+// where its value is infinite or NaN.  Its value is replaced by 0 with integer
+// operations on the x entry it multiplies (a compare of doubles would run on
+// the FP64 pipe); sums are never -0, so adding 0 * 0 leaves them as they are.
+__device__ __forceinline__ bool is_zero(double v)
+{
+    return ((__double2hiint(v) << 1) | __double2loint(v)) == 0;
+}
+
+template <int SIGMA, int VK, int AB, bool SKIP, class Src>
 __device__ __forceinline__ void compute_warp(const Src &src, const Smem<SIGMA, VK> &sm,
                                              int cw, int lane, uint64_t pol_x)
 {
@@ -528,7 +538,11 @@ __device__ __forceinline__ void compute_warp(const Src &src, const Smem<SIGMA, V
                 });
                 f32_odd = odd != 0u;
             } else {
-                chain([&](int j) { return (double)vst[c0 + j]; });
+                chain([&](int j) {
+                    if constexpr (SKIP && VK == VAL_F64)
+                        if (is_zero(xv[j])) return 0.0;
+                    return (double)vst[c0 + j];
+                });
             }
             if (sb && mask != 0u) head_row = r0;
         } else if (cnt > 0) {
@@ -561,7 +575,7 @@ __device__ __forceinline__ void compute_warp(const Src &src, const Smem<SIGMA, V
                 }
                 if (j < cnt) {
                     if (VK == VAL_PATTERN) sum += xv[j];
-                    else sum = fma((double)vst[c0 + j], xv[j], sum);
+                    else if (!SKIP || !is_zero(xv[j])) sum = fma((double)vst[c0 + j], xv[j], sum);
                 }
             }
             headv[t] = head_val;
@@ -788,8 +802,9 @@ __device__ __forceinline__ void epilogue_warp(const Src &src, const Smem<SIGMA, 
 template <int SIGMA, int VK>
 constexpr int min_ctas() { return (SIGMA == 11 && VK != VAL_F64) ? 5 : 1; }
 
-template <int SIGMA, int VK, int AB, class Src>
-__global__ void __launch_bounds__(CTA_THREADS, min_ctas<SIGMA, VK>()) tile_spmv_kernel(const Src a)
+template <int SIGMA, int VK, int AB, class Src, bool SKIP>
+__global__ void __launch_bounds__(CTA_THREADS, min_ctas<SIGMA, VK>())
+    tile_spmv_kernel(const Src src)
 {
     using L = Layout<SIGMA, VK>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -813,12 +828,23 @@ __global__ void __launch_bounds__(CTA_THREADS, min_ctas<SIGMA, VK>()) tile_spmv_
     // launched right behind the tile partition: the set-up above overlapped
     // its end; nothing in global memory is read before it has finished
     ptx::griddep_wait();
-    if (warp == NCW)
-        producer_warp<SIGMA, VK, Src>(a, sm, lane, ptx::policy_evict_first());
-    else if (warp > NCW)
-        epilogue_warp<SIGMA, VK, AB, Src>(a, sm, warp - NCW - 1, lane);
-    else
-        compute_warp<SIGMA, VK, AB, Src>(a, sm, warp, lane, ptx::policy_evict_last());
+    auto roles = [&](const Src &a) {
+        if (warp == NCW)
+            producer_warp<SIGMA, VK, Src>(a, sm, lane, ptx::policy_evict_first());
+        else if (warp > NCW)
+            epilogue_warp<SIGMA, VK, AB, Src>(a, sm, warp - NCW - 1, lane);
+        else
+            compute_warp<SIGMA, VK, AB, SKIP, Src>(a, sm, warp, lane, ptx::policy_evict_last());
+    };
+    if constexpr (SKIP) {
+        // col and val may hold more entries than the row pointer says (the
+        // x-zero filter drops them): the row pointer's count is what exists
+        Src a = src;
+        a.nnz = min(a.nnz, (long long)__ldg(a.rowptr + a.m));
+        roles(a);
+    } else {
+        roles(src);
+    }
 }
 
 // part[k] = number of rows r with rowptr[r+1] <= k*TILE (k = 1..ntiles-1);
@@ -843,6 +869,18 @@ __device__ __forceinline__ void own_tiles(int r, int b, int e, int ntiles, unsig
     for (; k <= k1 && k < (unsigned)ntiles; ++k) part[k] = r;
 }
 
+// Tiles that start at or past rowptr[m] (arrays longer than the row pointer
+// says) own no rows.
+__device__ __forceinline__ void own_no_rows(int m, const int *__restrict__ rowptr, int ntiles,
+                                            unsigned tile, int *__restrict__ part)
+{
+    if (blockIdx.x != 0) return;
+    const unsigned end = (unsigned)max(__ldg(rowptr + m), 0);
+    const unsigned long long k0 = ((unsigned long long)end + tile - 1) / tile;
+    for (unsigned long long k = max(k0, 1ull) + threadIdx.x; k < (unsigned)ntiles; k += blockDim.x)
+        part[k] = m;
+}
+
 __global__ void tile_partition_kernel(int m, long long nnz, int ntiles, long long tile,
                                       const int *__restrict__ rowptr, int *__restrict__ part)
 {
@@ -854,6 +892,7 @@ __global__ void tile_partition_kernel(int m, long long nnz, int ntiles, long lon
         part[0] = 0;
         part[ntiles] = m;
     }
+    own_no_rows(m, rowptr, ntiles, (unsigned)tile, part);
     for (int r = g; r < m; r += stride)
         own_tiles(r, __ldg(rowptr + r), __ldg(rowptr + r + 1), ntiles, (unsigned)tile, part);
 }
@@ -875,6 +914,7 @@ __global__ void tile_partition_quad_kernel(int m, int ntiles, long long tile,
     const long long nq = m / 4;
     const int4 *q4 = reinterpret_cast<const int4 *>(rowptr);
     const unsigned t32 = (unsigned)tile;
+    own_no_rows(m, rowptr, ntiles, t32, part);
     auto quad = [&](const int4 v, int next, long long r0) {
         own_tiles((int)r0, v.x, v.y, ntiles, t32, part);
         own_tiles((int)r0 + 1, v.y, v.z, ntiles, t32, part);
@@ -963,11 +1003,11 @@ constexpr int kNumSigmas = sizeof(kSigmas) / sizeof(kSigmas[0]);
 // sigma = 11, ~54 registers) would pass the limit again, so the request is
 // padded until the CTAs that fit stay within it (one CTA fewer), down to two
 // CTAs per SM.
-template <int SIGMA, int VK, int AB, class Src = TileArgs>
+template <int SIGMA, int VK, int AB, class Src = TileArgs, bool SKIP = false>
 int configure_shape(int *out_bps, size_t *out_smem)
 {
     using L = Layout<SIGMA, VK>;
-    auto kfn = tile_spmv_kernel<SIGMA, VK, AB, Src>;
+    auto kfn = tile_spmv_kernel<SIGMA, VK, AB, Src, SKIP>;
     constexpr int kMaxDev = 64;
     constexpr size_t kSmemLimit = size_t(195) * 1024;   // per SM, with the 1 KB per CTA
     static std::atomic<int> blocks_per_sm[kMaxDev];
@@ -1012,13 +1052,13 @@ int configure_shape(int *out_bps, size_t *out_smem)
     return SBLAS_OK;
 }
 
-template <int SIGMA, int VK, int AB, class Src = TileArgs>
+template <int SIGMA, int VK, int AB, class Src = TileArgs, bool SKIP = false>
 int launch_shape(const Src &a, cudaStream_t stream)
 {
-    auto kfn = tile_spmv_kernel<SIGMA, VK, AB, Src>;
+    auto kfn = tile_spmv_kernel<SIGMA, VK, AB, Src, SKIP>;
     int bps = 0;
     size_t smem = 0;
-    const int rc = configure_shape<SIGMA, VK, AB, Src>(&bps, &smem);
+    const int rc = configure_shape<SIGMA, VK, AB, Src, SKIP>(&bps, &smem);
     if (rc != SBLAS_OK) return rc;
     const int grid = min(a.ntiles, bps * device_num_sms());
     SBLAS_CUDA_TRY(launch_pdl(kfn, dim3(grid), dim3(CTA_THREADS), smem, stream, a));
@@ -1026,12 +1066,13 @@ int launch_shape(const Src &a, cudaStream_t stream)
     return SBLAS_OK;
 }
 
-template <int SIGMA, int VK>
+template <int SIGMA, int VK, bool SKIP = false>
 int launch_ab(const TileArgs &a, cudaStream_t stream)
 {
-    if (a.alpha == 1.0 && a.beta == 0.0) return launch_shape<SIGMA, VK, 0>(a, stream);
-    if (a.beta == 0.0) return launch_shape<SIGMA, VK, 1>(a, stream);
-    return launch_shape<SIGMA, VK, 2>(a, stream);
+    if (a.alpha == 1.0 && a.beta == 0.0)
+        return launch_shape<SIGMA, VK, 0, TileArgs, SKIP>(a, stream);
+    if (a.beta == 0.0) return launch_shape<SIGMA, VK, 1, TileArgs, SKIP>(a, stream);
+    return launch_shape<SIGMA, VK, 2, TileArgs, SKIP>(a, stream);
 }
 
 template <int SIGMA>
@@ -1282,7 +1323,8 @@ void set_test_stall(int on) { g_stall.store(on ? 1 : 0, std::memory_order_relaxe
 
 int launch_tile_spmv(int m, int n, long long nnz, double alpha, const void *val, int val_kind,
                      const int *rowptr, const int *col, const double *x, double beta, double *y,
-                     int sigma, void *work, cudaStream_t stream, bool analysed, bool reset_status)
+                     int sigma, void *work, cudaStream_t stream, bool analysed, bool reset_status,
+                     bool skip_zero_x)
 {
     if (m <= 0) return SBLAS_OK;
     if (nnz <= 0) return launch_scale_y(m, beta, y, stream);
@@ -1328,7 +1370,14 @@ int launch_tile_spmv(int m, int n, long long nnz, double alpha, const void *val,
     a.stall = g_stall.load(std::memory_order_relaxed);
     a.wait_ns = g_wait_ns.load(std::memory_order_relaxed);
     int rc = SBLAS_OK;
-    switch (sigma) {
+    if (skip_zero_x) {   // compiled for the default shape, FP64 values and pattern-only
+        if (sigma != 11 || (val_kind != VAL_F64 && val_kind != VAL_PATTERN)) {
+            set_error(SBLAS_ERR_UNSUPPORTED, "sparse x: sigma %d, value kind %d", sigma, val_kind);
+            return SBLAS_ERR_UNSUPPORTED;
+        }
+        rc = val_kind == VAL_F64 ? launch_ab<11, VAL_F64, true>(a, stream)
+                                 : launch_ab<11, VAL_PATTERN, true>(a, stream);
+    } else switch (sigma) {
     case 11: rc = launch_vk<11>(val_kind, a, stream); break;
     case 15: rc = launch_vk<15>(val_kind, a, stream); break;
     case 19: rc = launch_vk<19>(val_kind, a, stream); break;

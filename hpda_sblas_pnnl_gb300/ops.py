@@ -554,9 +554,31 @@ def spmspv(rowptr: torch.Tensor, col: torch.Tensor, val: torch.Tensor | None, x:
            kernel: int = KERNEL_MERGEPATH) -> torch.Tensor:
     """y = alpha*A'*x + beta*y with A' = A without the nonzeros whose x entry
     is zero, as spMspV_mgpu_v1 computes it (src/dspmv_mgpu_v1.cu:19-74), on
-    device arrays: the filter and the product both run on the GPU."""
-    orp, ocol, oval = csr_filter_x(rowptr, col, val, x)
-    return csrmv(orp, ocol, oval, x, y, alpha, beta, n=x.numel(), kernel=kernel)
+    device arrays: the filter is part of the product (sblas_dspmspv), so no
+    filtered matrix is made and nothing is read back."""
+    dev = _require_cuda(rowptr, col, val, x)
+    if val is not None and val.dtype != torch.float64:
+        raise TypeError("val must be float64 or None")
+    _require_dtype("rowptr", rowptr, torch.int32)
+    _require_dtype("col", col, torch.int32)
+    _require_dtype("x", x, torch.float64)
+    m = rowptr.numel() - 1
+    nnz = col.numel()
+    _require_len("val", val, nnz)
+    if _require_cuda(y) != dev:
+        raise ValueError("all tensors must be on one device")
+    _require_dtype("y", y, torch.float64)
+    if y.numel() != m:
+        raise ValueError("shape mismatch")
+    lib = _lib.load()
+    wb = workspace_bytes(nnz)
+    work = torch.empty(wb, dtype=torch.uint8, device=dev)
+    with torch.cuda.device(dev):
+        rc = lib.sblas_dspmspv(kernel, m, x.numel(), nnz, float(alpha), _ptr(val), _ptr(rowptr),
+                               _ptr(col), _ptr(x), float(beta), _ptr(y), _ptr(work), wb,
+                               _stream_ptr(dev))
+    _lib.check(rc)
+    return y
 
 
 def check_device(device: torch.device | None = None, clear: bool = True) -> None:

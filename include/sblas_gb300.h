@@ -286,6 +286,17 @@ SBLAS_API int sblas_csr_filter_x(int m, long long nnz, const int *rowptr, const 
                                  const double *val, const double *x, int *out_rowptr,
                                  int *out_col, double *out_val, void *work, size_t work_bytes,
                                  void *stream);
+/* y = alpha*A'*x + beta*y with A' = A without the nonzeros whose x entry is
+ * zero (spMspV_mgpu_v1 / _v2 on device arrays): the filter is taken inside
+ * the product, so infinite or NaN values at zeros of x stay out of y.  val:
+ * FP64, or NULL (pattern-only; kernels 2 and 3).  col and val may hold more
+ * than rowptr[m] entries (nnz of them).  work: as sblas_dcsrmv with sigma 0,
+ * required for kernels 2 and 3 (sblas_tile_workspace_bytes(nnz, 0), 256-byte
+ * aligned).  No allocation, no synchronisation: can be captured in a graph. */
+SBLAS_API int sblas_dspmspv(int kernel, int m, int n, long long nnz, double alpha,
+                            const double *val, const int *rowptr, const int *col,
+                            const double *x, double beta, double *y, void *work,
+                            size_t work_bytes, void *stream);
 /* dst[p] = src[perm[p]] for nnz values of the given kind (FP64 or FP32). */
 SBLAS_API int sblas_gather_values(long long nnz, int val_kind, const void *src, const int *perm,
                                   void *dst, void *stream);

@@ -78,3 +78,39 @@ def test_plan_picks_a_shape_for_every_size(sblas_lib, cuda, k, nnz):
     dval = op.grad_val(gy, x)
     assert rel_l2(dval.cpu().numpy(), O.csr_sddmm(m, m, rp, col, gy.cpu().numpy(),
                                                    x.cpu().numpy())) <= RTOL_L2
+
+
+@pytest.mark.parametrize("kernel", [1, 2, 3])
+@pytest.mark.parametrize("lengths", [[1], [0, 0, 1408, 0], [1407, 1, 1], [1409], [0] * 700 + [3],
+                                     [2, 0, 9000, 1, 0, 0, 40, 1500, 7] * 3], ids=str)
+@pytest.mark.parametrize("extra", [0, 1, 1408, 4000])
+def test_spmspv_leaves_out_zero_x(sblas_lib, cuda, kernel, lengths, extra):
+    """Zeros and negative zeros of x meet infinite and NaN values; rows that
+    cross tiles, empty rows, more rows than a tile holds; col and val longer
+    than the row pointer says."""
+    from hpda_sblas_pnnl_gb300 import ops
+    n = 300
+    (rp, col, val), (trp, _, _) = csr_of_lengths(lengths, n, 5, cuda)
+    m, nnz = len(lengths), int(rp[-1])
+    rng = np.random.default_rng(nnz)
+    x = rng.standard_normal(n)
+    x[rng.random(n) < 0.5] = 0.0
+    x[rng.random(n) < 0.1] = -0.0
+    dead = x[col] == 0.0
+    val[dead] = rng.choice([np.inf, -np.inf, np.nan, 2.0], int(dead.sum()))
+    y0 = rng.standard_normal(m)
+    orp, oc, ov = O.csr_filter_x(m, rp, col, val, x)
+    long_col = torch.from_numpy(np.concatenate([col, np.zeros(extra, np.int32)])).to(cuda)
+    long_val = torch.from_numpy(np.concatenate([val, np.full(extra, 3.0)])).to(cuda)
+    tx = torch.from_numpy(x).to(cuda)
+    for alpha, beta in ((1.0, 0.0), (1.5, 0.0), (1.5, -0.5)):
+        y = torch.from_numpy(y0).to(cuda)
+        ops.spmspv(trp, long_col, long_val, tx, y, alpha, beta, kernel=kernel)
+        ref = O.csr_spmv(m, n, orp, oc, ov, x, y0.copy(), alpha, beta)
+        assert rel_l2(y.cpu().numpy(), ref) <= RTOL_L2
+        if kernel == 1:
+            continue
+        y = torch.from_numpy(y0).to(cuda)
+        ops.spmspv(trp, long_col, None, tx, y, alpha, beta, kernel=kernel)
+        ref = O.csr_spmv(m, n, orp, oc, np.ones(len(oc)), x, y0.copy(), alpha, beta)
+        assert rel_l2(y.cpu().numpy(), ref) <= RTOL_L2
