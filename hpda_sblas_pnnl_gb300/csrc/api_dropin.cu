@@ -331,19 +331,19 @@ spmv_ret run_host(Call c)
     const double beta_eff = c.additive ? c.beta + 1.0 : c.beta;
     void *tile_work = nullptr;   // workspace of the tile launch, if one ran
     if (csc_direct && rows > 0) {
-        // the CSC product: the row-ordered structure by a stable bucket sort
-        // (inspector), then the values in row order and the tile kernel
+        // the CSC product: the entries in row order by a stable bucket sort
+        // (inspector), then the tile kernel
         const size_t wb = cscmv_workspace_bytes(m, n, nnz);
         void *w = device_scratch(6, wb);
         if (!w) {
             set_error(SBLAS_ERR_ALLOC, "%s: workspace allocation failed", c.name);
             return failed();
         }
-        if (launch_csc_analyse(m, n, nnz, d_ptr, d_idx, w, wb, false, st) != SBLAS_OK)
+        if (launch_csc_analyse(m, n, nnz, d_ptr, d_idx, d_val, w, wb, st) != SBLAS_OK)
             return failed();
         DROPIN_CUDA(cudaEventRecord(e2, st));   // the inspector counts as format work
-        if (launch_cscmv_analysed(m, n, nnz, c.alpha, d_val, d_x, beta_eff, d_y, w, wb, false,
-                                  st) != SBLAS_OK)
+        if (launch_cscmv_analysed(m, n, nnz, c.alpha, nullptr, d_x, beta_eff, d_y, w, wb, st) !=
+            SBLAS_OK)
             return failed();
         if (nnz > 0 && n > 0) tile_work = csc_tile_workspace(w, m, n, nnz);
     } else if (rows > 0) {

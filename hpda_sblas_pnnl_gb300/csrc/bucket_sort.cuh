@@ -1,69 +1,273 @@
-// Stable bucket scatter by one digit of an int key: the building block of
-// this library's sorts (own kernels; no library sort).
+// Stable bucket scatter by one digit of an int key: the step of this library's
+// least-significant-digit sorts (own kernels; no library sort).
 //
-// One pass over n entries, digit d(e) = (key(e) >> shift) & (nb - 1), nb <= 256:
-//   bucket_hist_kernel    per CTA tile (TILE entries): digit counts (shared-
-//                         memory counters), written digit-major: table[d * ntiles + t]
-//   exclusive scan        of the table (scan_* kernels): entry (d, t) becomes the
-//                         output position of tile t's first entry of digit d
-//   bucket_scatter_kernel per tile: stable ranks of its entries (every warp walks
-//                         its TILE / NW entries in order, ranking equal digits with
-//                         a warp match and counting in a warp-private shared
-//                         table), the tile sorted by digit in shared memory with
-//                         its payloads, then written out so that consecutive
-//                         threads write consecutive positions of one digit's run
-//                         (about TILE / nb entries): coalesced stores.
-//                         Every key and payload load of a tile is issued
-//                         before the first is used, and tiles are small
-//                         (~51 KB of shared memory, 64 registers per thread)
-//                         so that four CTAs per SM hide the memory latency.
+// One pass over n entries in tiles of T = 256 * ITER, digit
+// d(e) = (key(e) >> shift) & (nb - 1), nb <= 2048:
+//   bucket_hist_kernel    a CTA counts the digits of a chunk of consecutive
+//                         tiles in shared memory and writes, before each tile,
+//                         the counts so far: prefix[t][d] inside the chunk,
+//                         then the chunk's totals
+//   bucket_chunks_kernel  the chunk totals scanned over the chunks, per digit,
+//                         and the digits' totals
+//   bucket_scatter_kernel per tile: stable ranks of its entries (every warp
+//                         walks its 32 * ITER entries in order, finding equal
+//                         digits by ballots over the digit's bits and counting
+//                         in a warp-private shared table), then one array
+//                         after another is put into digit order in shared
+//                         memory and written out so that consecutive threads
+//                         write consecutive positions of one digit's run
+// Every table is digit-contiguous, so all its reads and writes are coalesced.
 // Entries keep their input order inside every digit (tiles in order, warps in
-// order inside a tile, entries in order inside a warp): a least-significant-
-// digit sequence of passes is a stable sort.  Counts are integers and
-// positions are computed, not claimed with atomics: every run produces the
-// same output.
+// order inside a tile, entries in order inside a warp).  Counts are integers
+// and positions are computed, not claimed with atomics: every run produces
+// the same output.
+//
+// Bound: the SM's store path, one request per 128-byte line that a warp's store
+// touches: three arrays in runs of T / nb = 4 entries are ~27 requests per 32
+// entries.  20M entries, 1024 digits, keys, columns and values: 234 us a pass
+// (a coalesced move of the same bytes 119 us, their HBM time 94 us).  Two
+// passes of up to 11 bits beat three of 8 all the same: 194 us each at 128
+// digits.  Equal digits by ballots rather than __match_any_sync, which takes a
+// warp's distinct values one after another: 312 -> 289 us in a copy of the
+// pass; CTAs of 512 threads (twice the warp-private tables): 326 us.
+// CSC to CSR, 20M entries, 1M rows: 890 -> 619 us; one product of a CSC matrix
+// with 4.5M entries: 275 -> 188 us.
 #pragma once
 
 #include <climits>
 
+#include "launch.cuh"
+#include "ptx.cuh"
 #include "sblas_internal.h"
 
 namespace sblas {
 namespace bsort {
+// The kernels here are launched behind one another with programmatic stream
+// serialisation and read what the kernel before wrote.  Those reads are plain
+// loads (no __restrict__, no __ldg): a load marked as reading constant memory
+// could be moved ahead of the wait for that kernel.
 // internal linkage: every translation unit that includes this header gets its
 // own copy of the kernels (no relocatable device code)
 namespace {
 
 constexpr int NW = 8;                   // warps per CTA
 constexpr int THREADS = NW * 32;
-constexpr int ITER = 8;                 // entries per lane per tile
-constexpr int WSPAN = 32 * ITER;        // entries of one warp in a tile (256)
-constexpr int TILE = NW * WSPAN;        // entries per CTA tile (2048)
-constexpr int MAXB = 256;               // digit values per pass (8-bit digits)
+constexpr int MAXB = 2048;              // digit values per pass (11-bit digits)
+constexpr int CHUNK_DIGITS = 32;        // digits per CTA of the chunk scan
 
-__host__ __device__ inline long long num_tiles(long long n) { return (n + TILE - 1) / TILE; }
+// Entries per thread of a pass over n entries: 16 (tiles of 4096, about four
+// entries per run at 1024 digits), or fewer where that would leave the three
+// CTAs that fit on each of the 152 SMs without a tile.
+inline int pass_iter(long long n) { return n >= (1LL << 22) ? 16 : n >= (1LL << 19) ? 8 : 4; }
+
+inline long long num_tiles(long long n, int iter)
+{
+    const long long t = (long long)THREADS * iter;
+    return (n + t - 1) / t;
+}
+
+// Tiles per chunk of the digit counts: about a thousand chunks.
+inline int chunk_tiles(long long ntiles)
+{
+    long long c = (ntiles + 1023) / 1024;
+    return (int)(c < 1 ? 1 : c);
+}
 
 __device__ __forceinline__ int digit_of(int key, int shift, int nb)
 {
     return (int)(((unsigned)key >> shift) & (unsigned)(nb - 1));
 }
 
-// ---- pass 1: digit counts per tile ----------------------------------------
-template <class Op>
-__global__ void __launch_bounds__(THREADS) bucket_hist_kernel(const Op op, long long n, int shift,
-                                                              int nb, int ntiles,
-                                                              int *__restrict__ table)
+// Width of a table row: the digits, or the eight that one thread scans.
+__host__ __device__ inline int table_width(int nb) { return nb < 8 ? 8 : nb; }
+
+// Ranks of this warp's entries among the equal digits before them (batch i,
+// then lane), counted in the warp's own table.  d[i] < 0: no entry.
+template <int ITER>
+__device__ __forceinline__ void rank_digits(const int (&d)[ITER], int bits,
+                                            unsigned short *mycnt, int lane, int (&rank)[ITER])
 {
+    const unsigned lt = (1u << lane) - 1u;
+#pragma unroll
+    for (int i = 0; i < ITER; ++i) {
+        const bool valid = d[i] >= 0;
+        unsigned peers = __ballot_sync(0xffffffffu, valid);
+        rank[i] = 0;
+        if (peers == 0u) continue;
+#pragma unroll
+        for (int b = 0; b < 11; ++b)
+            if (b < bits) {
+                const bool one = (d[i] >> b) & 1;
+                const unsigned m = __ballot_sync(0xffffffffu, one);
+                peers &= one ? m : ~m;
+            }
+        const int base = valid ? (int)mycnt[d[i]] : 0;
+        rank[i] = base + __popc(peers & lt);
+        __syncwarp();
+        if (valid && (peers & lt) == 0u) mycnt[d[i]] = (unsigned short)(base + __popc(peers));
+        __syncwarp();
+    }
+}
+
+__device__ __forceinline__ uint4 add_u16(uint4 a, uint4 b)
+{
+    return make_uint4(__vadd2(a.x, b.x), __vadd2(a.y, b.y), __vadd2(a.z, b.z), __vadd2(a.w, b.w));
+}
+__device__ __forceinline__ int sum_u16(uint4 v)
+{
+    const unsigned s = (v.x & 0xffffu) + (v.x >> 16) + (v.y & 0xffffu) + (v.y >> 16) +
+                       (v.z & 0xffffu) + (v.z >> 16) + (v.w & 0xffffu) + (v.w >> 16);
+    return (int)s;
+}
+// first[j] = at + the counts before the j-th of eight packed counts
+__device__ __forceinline__ void starts_u16(uint4 v, int at, int (&first)[8])
+{
+    const unsigned w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        first[2 * j] = at;
+        at += (int)(w[j] & 0xffffu);
+        first[2 * j + 1] = at;
+        at += (int)(w[j] >> 16);
+    }
+}
+__device__ __forceinline__ uint4 pack_u16(const int (&v)[8])
+{
+    return make_uint4((unsigned)v[0] | ((unsigned)v[1] << 16), (unsigned)v[2] | ((unsigned)v[3] << 16),
+                      (unsigned)v[4] | ((unsigned)v[5] << 16), (unsigned)v[6] | ((unsigned)v[7] << 16));
+}
+// Sum over the warps of the eight counts of digits 8t .. 8t + 7.
+template <int WARPS>
+__device__ __forceinline__ uint4 count_u16(const unsigned short *wcnt, int width, int t)
+{
+    uint4 s = make_uint4(0, 0, 0, 0);
+#pragma unroll 8
+    for (int k = 0; k < WARPS; ++k)
+        s = add_u16(s, reinterpret_cast<const uint4 *>(wcnt + k * width)[t]);
+    return s;
+}
+// The warps' counts of digits 8t .. 8t + 7 become running starts from `run`.
+template <int WARPS>
+__device__ __forceinline__ void warp_starts_u16(unsigned short *wcnt, int width, int t, uint4 run)
+{
+#pragma unroll 8
+    for (int k = 0; k < WARPS; ++k) {
+        uint4 *q = reinterpret_cast<uint4 *>(wcnt + k * width) + t;
+        const uint4 c = *q;
+        *q = run;
+        run = add_u16(run, c);
+    }
+}
+
+// ---- digit counts ----------------------------------------------------------
+template <int ITER>
+__global__ void __launch_bounds__(THREADS) bucket_hist_kernel(const int *key,
+                                                              long long n, int shift, int nb,
+                                                              int ntiles, int per_chunk,
+                                                              int *prefix,
+                                                              int *chunk_sum)
+{
+    constexpr int T = THREADS * ITER;
     __shared__ int cnt[MAXB];
-    for (int i = threadIdx.x; i < nb; i += THREADS) cnt[i] = 0;
+    ptx::griddep_launch_dependents();
+    const int width = table_width(nb);
+    for (int d = threadIdx.x; d < width; d += THREADS) cnt[d] = 0;
     __syncthreads();
-    const long long t0 = (long long)blockIdx.x * TILE;
-    const int len = (int)min((long long)TILE, n - t0);
-    for (int i = threadIdx.x; i < len; i += THREADS)
-        atomicAdd(&cnt[digit_of(op.key(t0 + i), shift, nb)], 1);
+    ptx::griddep_wait();
+    const int first = blockIdx.x * per_chunk, last = min(first + per_chunk, ntiles);
+    for (int t = first; t < last; ++t) {
+        const long long e0 = (long long)t * T + threadIdx.x;
+        int k[ITER];
+#pragma unroll
+        for (int i = 0; i < ITER; ++i)
+            k[i] = e0 + i * THREADS < n ? *(key + e0 + i * THREADS) : 0;
+        int *row = prefix + (long long)t * width;
+        for (int d = threadIdx.x; d < width; d += THREADS) row[d] = cnt[d];
+        __syncthreads();   // the counts so far are read before this tile's are added
+#pragma unroll
+        for (int i = 0; i < ITER; ++i)
+            if (e0 + i * THREADS < n) atomicAdd(&cnt[digit_of(k[i], shift, nb)], 1);
+        __syncthreads();
+    }
+    int *sum = chunk_sum + (long long)blockIdx.x * width;
+    for (int d = threadIdx.x; d < width; d += THREADS) sum[d] = cnt[d];
+}
+
+// Per digit: chunk_sum becomes the exclusive prefix over the chunks, total[d]
+// their sum.  A CTA takes 32 digits, a row of 32 threads a span of chunks.
+__global__ void __launch_bounds__(1024) bucket_chunks_kernel(int width, int nchunks,
+                                                             int *chunk_sum,
+                                                             int *total)
+{
+    __shared__ int part[32][33];
+    ptx::griddep_launch_dependents();
+    ptx::griddep_wait();
+    const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+    const int d = blockIdx.x * CHUNK_DIGITS + lane;
+    const int per = (nchunks + 31) / 32;
+    const int c0 = min(g * per, nchunks), c1 = min(c0 + per, nchunks);
+    int s = 0;
+    if (d < width) {
+#pragma unroll 8
+        for (int c = c0; c < c1; ++c) s += chunk_sum[(long long)c * width + d];
+    }
+    part[g][lane] = s;
     __syncthreads();
-    for (int d = threadIdx.x; d < nb; d += THREADS)
-        table[(long long)d * ntiles + blockIdx.x] = cnt[d];
+    // warp g scans the 32 spans of digit g of this CTA
+    int v = part[lane][g];
+    const int own = v;
+#pragma unroll
+    for (int k = 1; k < 32; k <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, v, k);
+        if (lane >= k) v += o;
+    }
+    part[lane][g] = v - own;
+    if (lane == 31 && blockIdx.x * CHUNK_DIGITS + g < width)
+        total[blockIdx.x * CHUNK_DIGITS + g] = v;
+    __syncthreads();
+    if (d < width) {
+        int p = part[g][lane];
+#pragma unroll 8
+        for (int c = c0; c < c1; ++c) {
+            const long long i = (long long)c * width + d;
+            const int x = chunk_sum[i];
+            chunk_sum[i] = p;
+            p += x;
+        }
+    }
+}
+
+// Exclusive scan over a CTA of THREADS threads of two sums at once.
+struct Two {
+    int a, b;
+};
+__device__ __forceinline__ Two block_scan_two(Two v)
+{
+    __shared__ int wa[NW], wb[NW];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    Two in = v;
+#pragma unroll
+    for (int k = 1; k < 32; k <<= 1) {
+        const int oa = __shfl_up_sync(0xffffffffu, v.a, k);
+        const int ob = __shfl_up_sync(0xffffffffu, v.b, k);
+        if (lane >= k) {
+            v.a += oa;
+            v.b += ob;
+        }
+    }
+    if (lane == 31) {
+        wa[w] = v.a;
+        wb[w] = v.b;
+    }
+    __syncthreads();
+    Two out{v.a - in.a, v.b - in.b};
+#pragma unroll
+    for (int k = 0; k < NW; ++k)
+        if (k < w) {
+            out.a += wa[k];
+            out.b += wb[k];
+        }
+    return out;
 }
 
 // ---- exclusive scan of int counts (sums < 2^31) ---------------------------
@@ -203,291 +407,342 @@ inline int exclusive_scan(const int *in, int *out, long long n, void *tmp, int *
     return SBLAS_OK;
 }
 
-// ---- pass 2: stable scatter ------------------------------------------------
-// What an entry carries besides its key: up to two ints and one double.
-struct Payload {
-    int a;
-    int b;
-    double d;
+// ---- stable scatter ---------------------------------------------------------
+// What a pass moves: the keys and up to two ints and one double per entry.
+// An output that is null is not carried.
+//   SEG   a is not read but is the segment (column of CSC, row of CSR) of the
+//         entry in ptr[0 .. nseg]
+//   IDX   b is not read but is the entry's own position
+//   POS   pos_out[e] receives entry e's output position
+struct Arrays {
+    const int *key_in = nullptr, *a_in = nullptr, *b_in = nullptr;
+    const double *d_in = nullptr;
+    const int *ptr = nullptr;
+    int nseg = 0;
+    int *key_out = nullptr, *a_out = nullptr, *b_out = nullptr;
+    double *d_out = nullptr;
+    int *pos_out = nullptr;
 };
 
-// Op: __device__ int key(long long e) const: the sort key of entry e;
-//     __device__ Payload load(State &st, long long e0, int lane, bool valid,
-//                             long long e) const: entry e's payload, called by
-//     all 32 lanes of a warp for the 32 consecutive entries e0 .. e0 + 31 (in
-//     increasing e0 per warp, so Op::State may carry a cursor);
-//     members key_out, a_out, b_out, d_out: the pass's outputs (a, b, d may
-//     be null: not carried);
-//     kPosOut: if true, the member pos_out receives every entry's output
-//     position at its input index (pos_out[e] = position of e); the
-//     payload's b must then be the entry's index e.
-template <class Op>
-__global__ void __launch_bounds__(THREADS, 4) bucket_scatter_kernel(const Op op, long long n,
-                                                                 int shift, int nb, int ntiles,
-                                                                 const int *__restrict__ table)
+// Shared memory of a scatter CTA: the staging buffer (8 bytes per entry),
+// the warps' digit counts and the digits' output offsets.
+template <int ITER>
+constexpr size_t scatter_smem_bytes(int width)
 {
-    extern __shared__ __align__(16) unsigned char bs_smem[];
-    double *st_d = reinterpret_cast<double *>(bs_smem);                  // [TILE]
-    int *st_key = reinterpret_cast<int *>(st_d + TILE);                  // [TILE]
-    int *st_a = st_key + TILE;                                           // [TILE]
-    int *st_b = st_a + TILE;                                             // [TILE]
-    unsigned short *loc = reinterpret_cast<unsigned short *>(st_b + TILE);   // [TILE]
-    unsigned short *wcnt = loc + TILE;                                   // [NW][MAXB]
-    int *gbase = reinterpret_cast<int *>(wcnt + NW * MAXB);              // [MAXB]
-    int *toff = gbase + MAXB;                                            // [MAXB]
-    __shared__ int wtot[NW];
+    return size_t(8) * THREADS * ITER + sizeof(unsigned short) * NW * (size_t)width +
+           sizeof(int) * (size_t)width;
+}
+
+// Segment of every entry of the tile [t0, t0 + cnt), into seg[0 .. cnt): the
+// largest s with ptr[s] <= entry.  The first and last segments are found by
+// the whole CTA (a 257-way search, three dependent loads for 4M segments),
+// each non-empty segment between them marks its first entry, and every warp
+// carries the marks forward over its entries (seg doubles as the marks).
+template <int ITER>
+__device__ __forceinline__ void tile_segments(const int *ptr, int nseg, long long t0,
+                                              int cnt, int *seg, int (&out)[ITER])
+{
+    constexpr int T = THREADS * ITER;
+    constexpr int WSPAN = 32 * ITER;
+    __shared__ int wlast[NW];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const long long t0 = (long long)blockIdx.x * TILE;
-    const long long wbeg = t0 + (long long)w * WSPAN;
-    const int cnt = (int)min((long long)TILE, n - t0);
-    for (int i = tid; i < NW * MAXB; i += THREADS) wcnt[i] = 0;
-    for (int d = tid; d < nb; d += THREADS)
-        gbase[d] = __ldg(table + (long long)d * ntiles + blockIdx.x);
-    // this warp's keys and payloads, every load in flight before the first
-    // is used (the kernel is bound by memory latency otherwise)
-    int kr[ITER];
-    Payload pl[ITER];
-    typename Op::State st{};
-#pragma unroll
-    for (int i = 0; i < ITER; ++i) {
-        const long long e = wbeg + (long long)i * 32 + lane;
-        kr[i] = e < n ? op.key(e) : 0;
+    const long long tl = t0 + cnt - 1;
+    for (int i = tid; i < T; i += THREADS) seg[i] = -1;
+    // segments holding entries t0 and tl: lo + (probes <= the entry) * step
+    int lo = 0, hi = nseg, lo2 = 0, hi2 = nseg;
+    while (hi - lo > 1 || hi2 - lo2 > 1) {   // the answers are in [lo, hi), [lo2, hi2)
+        const int st = (hi - lo + THREADS) / (THREADS + 1);
+        const int st2 = (hi2 - lo2 + THREADS) / (THREADS + 1);
+        const long long p = lo + (long long)(tid + 1) * st, p2 = lo2 + (long long)(tid + 1) * st2;
+        const bool le = p < hi && (long long)*(ptr + p) <= t0;
+        const bool le2 = p2 < hi2 && (long long)*(ptr + p2) <= tl;
+        const int c = __syncthreads_count(le), c2 = __syncthreads_count(le2);
+        lo += c * st;
+        hi = min(hi, lo + st);
+        lo2 += c2 * st2;
+        hi2 = min(hi2, lo2 + st2);
     }
-#pragma unroll
-    for (int i = 0; i < ITER; ++i) {
-        const long long e0 = wbeg + (long long)i * 32;
-        pl[i] = (e0 < n) ? op.load(st, e0, lane, e0 + lane < n, e0 + lane)   // warp-uniform
-                         : Payload{0, 0, 0.0};
+    __syncthreads();   // seg is cleared
+    for (long long s = (long long)lo + 1 + tid; s <= lo2; s += THREADS) {
+        const int b = *(ptr + s), e = *(ptr + s + 1);
+        if (e > b && b >= t0 && b <= tl) seg[b - t0] = (int)s;
     }
     __syncthreads();
-    unsigned short *mycnt = wcnt + w * MAXB;
-    const unsigned lt = (1u << lane) - 1u;
-    // ranks: entries of this warp in order (batch i, then lane)
+    int carry = -1;
 #pragma unroll
     for (int i = 0; i < ITER; ++i) {
-        const long long e = wbeg + (long long)i * 32 + lane;
-        const bool valid = e < n;
-        const int d = valid ? digit_of(kr[i], shift, nb) : -1 - lane;   // invalid: unique
-        const unsigned peers = __match_any_sync(0xffffffffu, d);
-        const int base = valid ? (int)mycnt[d] : 0;
-        __syncwarp();
-        if (valid) {
-            loc[w * WSPAN + i * 32 + lane] = (unsigned short)(base + __popc(peers & lt));
-            if ((peers & lt) == 0u) mycnt[d] = (unsigned short)(base + __popc(peers));
+        const int v = seg[w * WSPAN + i * 32 + lane];
+        const unsigned m = __ballot_sync(0xffffffffu, v >= 0) & (0xffffffffu >> (31 - lane));
+        const int got = __shfl_sync(0xffffffffu, v, m ? 31 - __clz(m) : 0);
+        out[i] = m ? got : carry;
+        carry = __shfl_sync(0xffffffffu, out[i], 31);
+    }
+    if (lane == 0) wlast[w] = carry;
+    __syncthreads();
+    int before = lo;
+#pragma unroll
+    for (int k = 0; k < NW; ++k)
+        if (k < w && wlast[k] >= 0) before = wlast[k];
+#pragma unroll
+    for (int i = 0; i < ITER; ++i) out[i] = out[i] >= 0 ? out[i] : before;
+}
+
+// Runs of a tile's digits: thread t takes digits 8t .. 8t + 7.  The warps'
+// counts become the slots of their first entries in the tile's digit order,
+// gpos[d] + slot is an entry's output position.
+__device__ __forceinline__ void tile_runs(unsigned short *wcnt, int *gpos, int width, int per_chunk,
+                                          const int *prefix,
+                                          const int *chunk_base,
+                                          const int *total)
+{
+    const int t = threadIdx.x;
+    const bool own = 8 * t < width;
+    uint4 c = make_uint4(0, 0, 0, 0);
+    int tot[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    Two sum{0, 0};
+    if (own) {
+        c = count_u16<NW>(wcnt, width, t);
+        const int4 lo = reinterpret_cast<const int4 *>(total)[2 * t];
+        const int4 hi = reinterpret_cast<const int4 *>(total)[2 * t + 1];
+        tot[0] = lo.x, tot[1] = lo.y, tot[2] = lo.z, tot[3] = lo.w;
+        tot[4] = hi.x, tot[5] = hi.y, tot[6] = hi.z, tot[7] = hi.w;
+        sum.a = sum_u16(c);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) sum.b += tot[j];
+    }
+    const Two at = block_scan_two(sum);
+    if (!own) return;
+    int first[8];
+    starts_u16(c, at.a, first);
+    warp_starts_u16<NW>(wcnt, width, t, pack_u16(first));
+    const int4 *row = reinterpret_cast<const int4 *>(prefix + (long long)blockIdx.x * width) + 2 * t;
+    const int4 *crow =
+        reinterpret_cast<const int4 *>(chunk_base + (long long)(blockIdx.x / per_chunk) * width) +
+        2 * t;
+    int b = at.b;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int4 r = row[h], c4 = crow[h];
+        const int before[4] = {r.x + c4.x, r.y + c4.y, r.z + c4.z, r.w + c4.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            gpos[8 * t + 4 * h + j] = b + before[j] - first[4 * h + j];
+            b += tot[4 * h + j];
         }
-        __syncwarp();
-    }
-    __syncthreads();
-    // per digit: the warps' offsets inside the digit's run, the run lengths
-    int total = 0;
-    if (tid < nb) {
-#pragma unroll
-        for (int k = 0; k < NW; ++k) {
-            const int c = wcnt[k * MAXB + tid];
-            wcnt[k * MAXB + tid] = (unsigned short)total;
-            total += c;
-        }
-    }
-    // exclusive scan of the run lengths over the digits: each run's start in
-    // the tile's sorted order (nb <= THREADS: one digit per thread)
-    int v = total;
-#pragma unroll
-    for (int k = 1; k < 32; k <<= 1) {
-        const int o = __shfl_up_sync(0xffffffffu, v, k);
-        if (lane >= k) v += o;
-    }
-    if (lane == 31) wtot[w] = v;
-    __syncthreads();
-    int before = 0;
-#pragma unroll
-    for (int k = 0; k < NW; ++k) before += (k < w) ? wtot[k] : 0;
-    if (tid < nb) toff[tid] = before + v - total;
-    __syncthreads();
-    // the tile in digit order, with its payloads, in shared memory
-    const bool ha = op.a_out != nullptr, hd = op.d_out != nullptr;
-    const bool hb = op.b_out != nullptr || Op::kPosOut;
-#pragma unroll
-    for (int i = 0; i < ITER; ++i) {
-        const long long e = wbeg + (long long)i * 32 + lane;
-        if (e < n) {
-            const int d = digit_of(kr[i], shift, nb);
-            const int slot = toff[d] + mycnt[d] + loc[w * WSPAN + i * 32 + lane];
-            st_key[slot] = kr[i];
-            if (ha) st_a[slot] = pl[i].a;
-            if (hb) st_b[slot] = pl[i].b;
-            if (hd) st_d[slot] = pl[i].d;
-        }
-    }
-    __syncthreads();
-    // write-out: consecutive slots of one digit go to consecutive positions
-    for (int j = tid; j < cnt; j += THREADS) {
-        const int k = st_key[j];
-        const int d = digit_of(k, shift, nb);
-        const long long pos = (long long)gbase[d] + (j - toff[d]);
-        if (op.key_out) op.key_out[pos] = k;
-        if (ha) op.a_out[pos] = st_a[j];
-        if (op.b_out) op.b_out[pos] = st_b[j];
-        if (hd) op.d_out[pos] = st_d[j];
-        if constexpr (Op::kPosOut) op.pos_out[st_b[j]] = (int)pos;   // inside the tile's span
     }
 }
 
-inline size_t scatter_smem_bytes()
+template <bool SEG, bool IDX, bool POS, int ITER>
+__global__ void __launch_bounds__(THREADS, 3) bucket_scatter_kernel(
+    const Arrays op, long long n, int shift, int nb, int bits, int per_chunk,
+    const int *prefix, const int *chunk_base,
+    const int *total)
 {
-    return (sizeof(double) + 3 * sizeof(int) + sizeof(unsigned short)) * TILE +
-           sizeof(unsigned short) * NW * MAXB + 2 * sizeof(int) * MAXB;
+    constexpr int T = THREADS * ITER;
+    constexpr int WSPAN = 32 * ITER;
+    extern __shared__ __align__(16) unsigned char bs_smem[];
+    const int width = table_width(nb);
+    double *buf = reinterpret_cast<double *>(bs_smem);                        // [T]
+    int *buf_i = reinterpret_cast<int *>(buf);
+    unsigned short *wcnt = reinterpret_cast<unsigned short *>(buf + T);       // [NW][width]
+    int *gpos = reinterpret_cast<int *>(wcnt + NW * width);                   // [width]
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const long long t0 = (long long)blockIdx.x * T;
+    const int cnt = (int)min((long long)T, n - t0);
+    const int mine = w * WSPAN + lane;       // this thread's entries: mine + 32 i
+    ptx::griddep_launch_dependents();
+    for (int i = tid; i < NW * width / 8; i += THREADS)
+        reinterpret_cast<uint4 *>(wcnt)[i] = make_uint4(0, 0, 0, 0);
+    ptx::griddep_wait();
+    int key[ITER];
+#pragma unroll
+    for (int i = 0; i < ITER; ++i)
+        key[i] = mine + 32 * i < cnt ? *(op.key_in + t0 + mine + 32 * i) : 0;
+    __syncthreads();
+    unsigned short *mycnt = wcnt + w * width;
+    int slot[ITER];
+    {
+        int d[ITER];
+#pragma unroll
+        for (int i = 0; i < ITER; ++i)
+            d[i] = mine + 32 * i < cnt ? digit_of(key[i], shift, nb) : -1;
+        rank_digits<ITER>(d, bits, mycnt, lane, slot);
+    }
+    __syncthreads();
+    tile_runs(wcnt, gpos, width, per_chunk, prefix, chunk_base, total);
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < ITER; ++i)
+        if (mine + 32 * i < cnt) {
+            const int d = digit_of(key[i], shift, nb);
+            slot[i] += mycnt[d];
+            if constexpr (POS) op.pos_out[t0 + mine + 32 * i] = gpos[d] + slot[i];
+            buf_i[slot[i]] = key[i];
+        }
+    __syncthreads();
+    // output position of the tile's j-th entry in digit order, j = tid + THREADS i
+    int pos[ITER];
+#pragma unroll
+    for (int i = 0; i < ITER; ++i) {
+        const int j = tid + THREADS * i;
+        pos[i] = 0;
+        if (j < cnt) {
+            const int k = buf_i[j];
+            pos[i] = gpos[digit_of(k, shift, nb)] + j;
+            if (op.key_out) op.key_out[pos[i]] = k;
+        }
+    }
+    if (op.d_out) {
+        double v[ITER];
+#pragma unroll
+        for (int i = 0; i < ITER; ++i)
+            v[i] = mine + 32 * i < cnt ? *(op.d_in + t0 + mine + 32 * i) : 0.0;
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < ITER; ++i)
+            if (mine + 32 * i < cnt) buf[slot[i]] = v[i];
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < ITER; ++i)
+            if (tid + THREADS * i < cnt) op.d_out[pos[i]] = buf[tid + THREADS * i];
+    }
+    if (op.a_out) {
+        int v[ITER];
+        if constexpr (SEG) {
+            __syncthreads();
+            tile_segments<ITER>(op.ptr, op.nseg, t0, cnt, buf_i, v);
+        } else {
+#pragma unroll
+            for (int i = 0; i < ITER; ++i)
+                v[i] = mine + 32 * i < cnt ? *(op.a_in + t0 + mine + 32 * i) : 0;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < ITER; ++i)
+            if (mine + 32 * i < cnt) buf_i[slot[i]] = v[i];
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < ITER; ++i)
+            if (tid + THREADS * i < cnt) op.a_out[pos[i]] = buf_i[tid + THREADS * i];
+    }
+    if (op.b_out) {
+        int v[ITER];
+#pragma unroll
+        for (int i = 0; i < ITER; ++i) {
+            const int e = mine + 32 * i;
+            v[i] = IDX ? (int)(t0 + e) : e < cnt ? *(op.b_in + t0 + e) : 0;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < ITER; ++i)
+            if (mine + 32 * i < cnt) buf_i[slot[i]] = v[i];
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < ITER; ++i)
+            if (tid + THREADS * i < cnt) op.b_out[pos[i]] = buf_i[tid + THREADS * i];
+    }
 }
 
-// Table bytes (counts / positions) and scan scratch of one pass over n entries.
-inline size_t pass_table_bytes(long long n, int nb)
+// ---- one pass ----------------------------------------------------------------
+// Scratch: prefix [tiles][nb] | chunk bases [chunks][nb] | totals [nb].
+struct PassTables {
+    int *prefix = nullptr, *chunk_base = nullptr, *total = nullptr;
+    long long tiles = 0;
+    int per_chunk = 1;
+    long long chunks = 0;
+    size_t bytes = 0;
+};
+
+inline PassTables pass_tables(long long n, int nb, int iter, void *work)
 {
-    return sizeof(int) * (size_t)nb * (size_t)(num_tiles(n) > 0 ? num_tiles(n) : 1);
-}
-inline size_t pass_work_bytes(long long n, int nb)
-{
-    const size_t t = (pass_table_bytes(n, nb) + 255) & ~size_t(255);
-    return t + ((scan_tmp_bytes((long long)nb * num_tiles(n)) + 255) & ~size_t(255));
+    PassTables t;
+    t.tiles = num_tiles(n > 0 ? n : 1, iter);
+    t.per_chunk = chunk_tiles(t.tiles);
+    t.chunks = (t.tiles + t.per_chunk - 1) / t.per_chunk;
+    auto up = [](size_t v) { return (v + 255) & ~size_t(255); };
+    const size_t row = 4 * (size_t)table_width(nb);
+    const size_t p = up(row * (size_t)t.tiles), c = up(row * (size_t)t.chunks);
+    unsigned char *w = static_cast<unsigned char *>(work);
+    t.prefix = reinterpret_cast<int *>(w);
+    t.chunk_base = reinterpret_cast<int *>(w + p);
+    t.total = reinterpret_cast<int *>(w + p + c);
+    t.bytes = p + c + up(row);
+    return t;
 }
 
-// One stable pass: entries of `op` scattered by digit (key >> shift) & (nb-1).
-// work: pass_work_bytes(n, nb) bytes.  Stream-ordered.
-template <class Op>
-int scatter_pass(const Op &op, long long n, int shift, int nb, void *work, cudaStream_t stream)
+inline size_t pass_work_bytes(long long n, int nb, int iter) { return pass_tables(n, nb, iter, nullptr).bytes; }
+inline size_t pass_work_bytes(long long n, int nb) { return pass_work_bytes(n, nb, pass_iter(n)); }
+
+inline int bits_for(int nb)   // bits of a digit in [0, nb)
+{
+    int b = 0;
+    while ((1 << b) < nb) ++b;
+    return b;
+}
+
+// Digit counts of a pass (the first two kernels).
+template <int ITER>
+int count_digits(const int *key, long long n, int shift, int nb, const PassTables &t,
+                 cudaStream_t stream)
+{
+    SBLAS_CUDA_TRY(launch_pdl(bucket_hist_kernel<ITER>, dim3((unsigned)t.chunks), dim3(THREADS), 0,
+                              stream, key, n, shift, nb, (int)t.tiles, t.per_chunk, t.prefix,
+                              t.chunk_base));
+    const int width = table_width(nb);
+    SBLAS_CUDA_TRY(launch_pdl(bucket_chunks_kernel,
+                              dim3((width + CHUNK_DIGITS - 1) / CHUNK_DIGITS), dim3(1024), 0,
+                              stream, width, (int)t.chunks, t.chunk_base, t.total));
+    return SBLAS_OK;
+}
+
+// A kernel's dynamic shared memory and the largest carveout: these kernels'
+// loads stream, nothing they read is reused through L1.
+template <class K>
+int allow_smem(K kfn, size_t bytes)
+{
+    SBLAS_CUDA_TRY(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    SBLAS_CUDA_TRY(cudaFuncSetAttribute(kfn, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                        (int)cudaSharedmemCarveoutMaxShared));
+    return SBLAS_OK;
+}
+
+template <bool SEG, bool IDX, bool POS, int ITER>
+int scatter_pass_iter(const Arrays &op, long long n, int shift, int nb, void *work,
+                      cudaStream_t stream)
 {
     if (n <= 0) return SBLAS_OK;
     if (nb < 1 || nb > MAXB || (nb & (nb - 1)) != 0) {
         set_error(SBLAS_ERR_ARG, "bucket pass: %d buckets", nb);
         return SBLAS_ERR_ARG;
     }
-    const long long nt = num_tiles(n);
-    if (nt > INT_MAX / MAXB) {
-        set_error(SBLAS_ERR_ARG, "bucket pass over %lld entries too large", n);
-        return SBLAS_ERR_ARG;
-    }
-    int *table = static_cast<int *>(work);
-    void *tmp = static_cast<unsigned char *>(work) + ((pass_table_bytes(n, nb) + 255) & ~size_t(255));
-    static_assert(TILE <= 65536, "tile offsets are 16-bit");
-    bucket_hist_kernel<Op><<<(unsigned)nt, THREADS, 0, stream>>>(op, n, shift, nb, (int)nt, table);
-    SBLAS_CUDA_TRY(cudaGetLastError());
-    const int rc = exclusive_scan(table, table, (long long)nb * nt, tmp, nullptr, stream);
+    const PassTables t = pass_tables(n, nb, ITER, work);
+    static_assert(THREADS * ITER <= 65535, "tile offsets are 16-bit");
+    int rc = count_digits<ITER>(op.key_in, n, shift, nb, t, stream);
     if (rc != SBLAS_OK) return rc;
-    auto kfn = bucket_scatter_kernel<Op>;
-    const size_t smem = scatter_smem_bytes();
-    SBLAS_CUDA_TRY(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)smem));
-    // four CTAs per SM (~208 KB): the largest shared-memory carveout; this
-    // kernel's loads stream, nothing it reads is reused through L1
-    SBLAS_CUDA_TRY(cudaFuncSetAttribute(kfn, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                        (int)cudaSharedmemCarveoutMaxShared));
-    kfn<<<(unsigned)nt, THREADS, smem, stream>>>(op, n, shift, nb, (int)nt, table);
-    SBLAS_CUDA_TRY(cudaGetLastError());
+    auto kfn = bucket_scatter_kernel<SEG, IDX, POS, ITER>;
+    rc = allow_smem(kfn, scatter_smem_bytes<ITER>(MAXB));
+    if (rc != SBLAS_OK) return rc;
+    SBLAS_CUDA_TRY(launch_pdl(kfn, dim3((unsigned)t.tiles), dim3(THREADS),
+                              scatter_smem_bytes<ITER>(table_width(nb)), stream, op, n, shift,
+                              nb, bits_for(nb), t.per_chunk, t.prefix, t.chunk_base, t.total));
     return SBLAS_OK;
 }
 
-// ---- segment of an entry in a compressed pointer array --------------------
-// ptr[0..nseg] (ptr[0] = 0, ptr[nseg] = entries, nondecreasing): the segment
-// (column of CSC, row of CSR) of entry e is the largest s with ptr[s] <= e.
-// A warp walking increasing batches e0 .. e0 + 31 keeps the segment of its
-// last batch in `cur` (-1 before the first): every batch then loads the 32
-// segment starts after it (coalesced) and each lane counts those <= its
-// entry with a 5-step shuffle search; runs of more than 32 short or empty
-// segments take further rounds.
-struct SegCursor {
-    int cur = -1;
-};
-
-__device__ __forceinline__ int segment_of(const int *__restrict__ ptr, int nseg, SegCursor &c,
-                                          long long e0, int lane, bool valid, long long e)
+// One stable pass: the entries of `op` scattered by digit
+// (key >> shift) & (nb-1).  work: pass_work_bytes(n, nb) bytes.  Stream-ordered.
+template <bool SEG, bool IDX>
+int scatter_pass(const Arrays &op, long long n, int shift, int nb, void *work,
+                 cudaStream_t stream)
 {
-    if (c.cur < 0) {
-        int lo = 0, hi = nseg - 1;   // largest s with ptr[s] <= e0 (warp-uniform)
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if ((long long)__ldg(ptr + mid) <= e0) lo = mid; else hi = mid - 1;
-        }
-        c.cur = lo;
+    switch (pass_iter(n)) {
+    case 16: return scatter_pass_iter<SEG, IDX, false, 16>(op, n, shift, nb, work, stream);
+    case 8: return scatter_pass_iter<SEG, IDX, false, 8>(op, n, shift, nb, work, stream);
+    default: return scatter_pass_iter<SEG, IDX, false, 4>(op, n, shift, nb, work, stream);
     }
-    const int ev = valid ? (int)e : INT_MIN;   // invalid lanes are found at once
-    int base = c.cur, seg = c.cur;
-    bool found = !valid;
-    for (;;) {
-        const int idx = base + 1 + lane;
-        const int st = idx <= nseg ? __ldg(ptr + idx) : INT_MAX;
-        int pos = 0;   // number of the 32 starts <= ev
-#pragma unroll
-        for (int b = 16; b > 0; b >>= 1) {
-            const int v = __shfl_sync(0xffffffffu, st, pos + b - 1);
-            if (v <= ev) pos += b;
-        }
-        const int v31 = __shfl_sync(0xffffffffu, st, 31);
-        if (pos == 31 && v31 <= ev) pos = 32;
-        if (!found && pos < 32) {
-            seg = base + pos;
-            found = true;
-        }
-        if (__all_sync(0xffffffffu, found)) break;
-        base += 32;
-    }
-    c.cur = __shfl_sync(0xffffffffu, valid ? seg : c.cur, 31);
-    return seg < nseg ? seg : nseg - 1;   // a malformed pointer never indexes past it
 }
 
-// ---- operations of the sorts ------------------------------------------------
-// Moves (key, a, b, d) from arrays to the pass's output positions; any of
-// a, b, d may be absent (null input and output).
-struct MoveOp {
-    const int *key_in;
-    const int *a_in;
-    const int *b_in;
-    const double *d_in;
-    int *key_out;
-    int *a_out;
-    int *b_out;
-    double *d_out;
-    static constexpr bool kPosOut = false;
-    struct State {};
-    __device__ int key(long long e) const { return __ldg(key_in + e); }
-    __device__ Payload load(State &, long long, int, bool valid, long long e) const
-    {
-        Payload p{0, 0, 0.0};
-        if (valid) {
-            if (a_in) p.a = __ldg(a_in + e);
-            if (b_in) p.b = __ldg(b_in + e);
-            if (d_in) p.d = __ldg(d_in + e);
-        }
-        return p;
-    }
-};
-
-// A compressed matrix's entries keyed by their index array (CSC: the row of
-// every entry), carrying the segment each entry belongs to (CSC: its column)
-// as `a`, the entry's own position as `b` and its value as `d`, as the
-// outputs ask.
-struct SegmentOp {
-    const int *key_in;
-    const int *ptr;      // segment pointer, nseg + 1 entries
-    int nseg;
-    const double *d_in;  // values, or null
-    int *key_out;
-    int *a_out;          // segment of the entry, or null
-    int *b_out;          // position of the entry, or null
-    double *d_out;
-    static constexpr bool kPosOut = false;
-    struct State {
-        SegCursor c;
-    };
-    __device__ int key(long long e) const { return __ldg(key_in + e); }
-    __device__ Payload load(State &st, long long e0, int lane, bool valid, long long e) const
-    {
-        Payload p{0, (int)e, 0.0};
-        if (a_out) p.a = segment_of(ptr, nseg, st.c, e0, lane, valid, e);
-        if (valid && d_in) p.d = __ldg(d_in + e);
-        return p;
-    }
-};
-
 // Digit widths of a least-significant-digit sort of keys in [0, key_bound):
-// as few passes as digits of at most 8 bits allow, equal widths.
+// as few passes as digits of at most 11 bits allow, equal widths.
 struct LsdPlan {
     int passes;
     int width;
@@ -496,7 +751,7 @@ inline LsdPlan lsd_plan(long long key_bound)
 {
     int bits = 1;
     while (bits < 31 && (1LL << bits) < key_bound) ++bits;
-    const int passes = (bits + 7) / 8;
+    const int passes = (bits + 10) / 11;
     return LsdPlan{passes, (bits + passes - 1) / passes};
 }
 

@@ -10,8 +10,8 @@
 //     pointer entries of the rows in between);
 //   * sorts (CSC -> CSR, A -> A^T, the COO sorts): a stable least-significant-
 //     digit sort by the row (or column) index, digits of at most 11 bits
-//     (bucket_sort.cuh: per-tile digit counts, an exclusive scan, a stable
-//     scatter): two passes for keys below 4M, three up to 2^31.  The first
+//     (bucket_sort.cuh: digit counts, a stable scatter): two passes for keys
+//     up to 2^22, three up to 2^31.  The first
 //     pass derives what the entries carry from the source (a CSC entry's
 //     column from the column pointer, an entry's own position), so no
 //     permutation has to be applied afterwards; stability keeps the second
@@ -168,13 +168,13 @@ ArraySet array_set(unsigned char *p, long long n, bool has_a, bool has_b, bool h
     return s;
 }
 
-// Stable sort of n entries by key in [0, key_bound).  Pass 1 reads through
-// `first` (its outputs are set here); later passes move the arrays; the last
-// pass writes `out` (out.key required; out.a / out.b / out.d as the first
-// operation carries them).
-template <class FirstOp>
-int lsd_sort(FirstOp first, long long n, long long key_bound, const ArraySet &out, void *work,
-             size_t work_bytes, cudaStream_t stream)
+// Stable sort of n entries by key in [0, key_bound).  Pass 1 reads `first`
+// (its outputs are set here; SEG and IDX as in bsort::Arrays); later passes
+// move the arrays; the last pass writes `out` (out.key required; out.a /
+// out.b / out.d as the first pass carries them).
+template <bool SEG, bool IDX>
+int lsd_sort(const bsort::Arrays &first, long long n, long long key_bound, const ArraySet &out,
+             void *work, size_t work_bytes, cudaStream_t stream)
 {
     if (n <= 0) return SBLAS_OK;
     const bool has_a = out.a != nullptr, has_b = out.b != nullptr, has_d = out.d != nullptr;
@@ -189,19 +189,21 @@ int lsd_sort(FirstOp first, long long n, long long key_bound, const ArraySet &ou
     const int nb = 1 << L.width;
     for (int p = 0; p < L.passes; ++p) {
         const ArraySet &dst = (p == L.passes - 1) ? out : tmp[p % 2];
-        int rc;
-        if (p == 0) {
-            FirstOp op = first;
-            op.key_out = dst.key;
-            op.a_out = dst.a;
-            op.b_out = dst.b;
-            op.d_out = dst.d;
-            rc = bsort::scatter_pass(op, n, 0, nb, w, stream);
-        } else {
+        bsort::Arrays op = first;
+        if (p > 0) {
             const ArraySet &src = tmp[(p - 1) % 2];
-            bsort::MoveOp op{src.key, src.a, src.b, src.d, dst.key, dst.a, dst.b, dst.d};
-            rc = bsort::scatter_pass(op, n, p * L.width, nb, w, stream);
+            op = bsort::Arrays();
+            op.key_in = src.key;
+            op.a_in = src.a;
+            op.b_in = src.b;
+            op.d_in = src.d;
         }
+        op.key_out = dst.key;
+        op.a_out = dst.a;
+        op.b_out = dst.b;
+        op.d_out = dst.d;
+        const int rc = p == 0 ? bsort::scatter_pass<SEG, IDX>(op, n, 0, nb, w, stream)
+                              : bsort::scatter_pass<false, false>(op, n, p * L.width, nb, w, stream);
         if (rc != SBLAS_OK) return rc;
     }
     return SBLAS_OK;
@@ -231,14 +233,17 @@ int launch_csc_to_csr(int m, int n, long long nnz, const double *csc_val, const 
         return SBLAS_ERR_ARG;
     }
     unsigned char *w = static_cast<unsigned char *>(work);
+    // the CSC arrays: key = row, a = column (from the column pointer), d = value
+    bsort::Arrays first;
+    first.key_in = csc_row;
+    first.ptr = csc_colptr;
+    first.nseg = n;
+    first.d_in = csc_val;
     ArraySet out;
     out.key = reinterpret_cast<int *>(w);   // the rows, sorted: the row pointer's source
     out.a = csr_col;
     out.d = csr_val;
-    // pass 1 reads the CSC arrays: key = row, a = column (from the column
-    // pointer), d = value
-    bsort::SegmentOp first{csc_row, csc_colptr, n, csc_val, nullptr, nullptr, nullptr, nullptr};
-    const int rc = lsd_sort(first, nnz, m, out, w + al256(4 * (size_t)nnz),
+    const int rc = lsd_sort<true, false>(first, nnz, m, out, w + al256(4 * (size_t)nnz),
                             work_bytes - al256(4 * (size_t)nnz), stream);
     if (rc != SBLAS_OK) return rc;
     return launch_coo_rows_to_rowptr(m, nnz, out.key, csr_rowptr, stream);
@@ -258,8 +263,11 @@ int launch_coo_sort(int key_bound, long long nnz, const int *keys, const int *ot
     out.key = keys_out;
     out.a = other_out;
     out.d = val_out;
-    bsort::MoveOp first{keys, other, nullptr, val, nullptr, nullptr, nullptr, nullptr};
-    return lsd_sort(first, nnz, key_bound, out, work, work_bytes, stream);
+    bsort::Arrays first;
+    first.key_in = keys;
+    first.a_in = other;
+    first.d_in = val;
+    return lsd_sort<false, false>(first, nnz, key_bound, out, work, work_bytes, stream);
 }
 
 namespace {
@@ -308,13 +316,16 @@ int launch_csr_transpose(int m, int n, long long nnz, const int *rowptr, const i
         return SBLAS_ERR_ARG;
     }
     unsigned char *w = static_cast<unsigned char *>(work);
+    bsort::Arrays first;
+    first.key_in = col;
+    first.ptr = rowptr;
+    first.nseg = m;
     ArraySet out;
     out.key = reinterpret_cast<int *>(w);   // the columns, sorted: A^T's row pointer source
     out.a = t_col;                          // the row of A holding the entry
     out.b = perm;                           // the entry's position in A
     // stable by column: the entries of one column keep their row order
-    bsort::SegmentOp first{col, rowptr, m, nullptr, nullptr, nullptr, nullptr, nullptr};
-    const int rc = lsd_sort(first, nnz, n, out, w + al256(4 * (size_t)nnz),
+    const int rc = lsd_sort<true, true>(first, nnz, n, out, w + al256(4 * (size_t)nnz),
                             work_bytes - al256(4 * (size_t)nnz), stream);
     if (rc != SBLAS_OK) return rc;
     return launch_coo_rows_to_rowptr(n, nnz, out.key, t_rowptr, stream);

@@ -12,10 +12,12 @@
 //   executor   the values in row order, then the CSR tile kernel: its
 //              segmented sums and carry fix-up in a fixed order, no atomics,
 //              bit-reproducible.
-// Two ways to put the values into row order:
-//   direct     out[p] = val[perm[p]]: one random read of every value from
-//              DRAM (the values do not fit in L2), used by the one-shot
-//              product, whose inspector runs on every call;
+// Ways to put the values into row order:
+//   sorted     the one-shot product, whose inspector runs on every call, lets
+//              the sort carry the values instead of the positions (a gather by
+//              position afterwards cost 24 us more on 4.5M entries);
+//   direct     out[p] = val[perm[p]], for an analysed pattern of one bucket
+//              (its values stay in L2);
 //   staged     for an analysed pattern reused many times (sblas_csc_analyse):
 //              the row-order positions are cut into buckets of 2^bits
 //              (8 MB of values).  The inspector adds two index arrays:
@@ -43,6 +45,8 @@ size_t al256(size_t v) { return (v + 255) & ~size_t(255); }
 
 constexpr int kCscSigma = 11;     // tile shape of the executor (the library default)
 constexpr int kStageBits = 20;    // staging bucket: 2^20 row positions (8 MB of values)
+constexpr int kStageBuckets = 256;   // at most (the bucket pass's digit values)
+constexpr int kStageIter = 8;     // entries per thread of the staging pass's tiles
 
 // Staging buckets of a matrix: nb is a power of two (the digit mask of the
 // bucket pass), used = the buckets that hold entries; used == 1: no staging.
@@ -54,7 +58,7 @@ StagePlan stage_plan(long long nnz)
 {
     StagePlan s{kStageBits, 1, 1};
     if (nnz <= 1) return s;
-    while (((nnz - 1) >> s.bits) >= bsort::MAXB) ++s.bits;
+    while (((nnz - 1) >> s.bits) >= kStageBuckets) ++s.bits;
     s.used = (int)(((nnz - 1) >> s.bits) + 1);
     while (s.nb < s.used) s.nb <<= 1;
     return s;
@@ -70,7 +74,7 @@ struct CscLayout {
     size_t rowptr, col, perm, dst, runs, val, tile, scratch, total;
 };
 
-long long stage_tiles(long long nnz) { return bsort::num_tiles(nnz); }
+long long stage_tiles(long long nnz) { return bsort::num_tiles(nnz, kStageIter); }
 
 CscLayout csc_layout(int m, int n, long long nnz)
 {
@@ -87,9 +91,10 @@ CscLayout csc_layout(int m, int n, long long nnz)
     L.val = L.runs + (staged ? al256(4 * nruns) + al256(2 * nruns) : 0);
     L.tile = L.val + al256(8 * nn);
     L.scratch = L.tile + al256(tile_workspace_bytes(nnz, kCscSigma));
-    size_t scratch = al256(csr_transpose_workspace_bytes(n, m, nnz));
+    size_t scratch = al256(std::max(csr_transpose_workspace_bytes(n, m, nnz),
+                                    csc_to_csr_workspace_bytes(m, n, nnz)));
     if (staged) {
-        const size_t inspect = 2 * al256(4 * nn) + al256(bsort::pass_work_bytes(nnz, sp.nb));
+        const size_t inspect = 2 * al256(4 * nn) + al256(bsort::pass_work_bytes(nnz, sp.nb, kStageIter));
         scratch = std::max(scratch, std::max(inspect, al256(8 * nn)));
     }
     L.total = L.scratch + scratch;
@@ -130,13 +135,13 @@ __global__ void __launch_bounds__(MOVE_THREADS) gather_values_kernel(long long n
 }
 
 // The staging scatter, stage[dst[q]] = val[q], one CTA per tile of
-// bsort::TILE CSC entries: the tiles of the staging pass that made dst, so
+// STAGE_TILE CSC entries: the tiles of the staging pass that made dst, so
 // the tile's entries of one bucket hold consecutive slots, from the run's
 // first slot on (runs, kept by the inspector).  The tile is regrouped in
 // shared memory by bucket (slot = the run's offset in the tile + dst - the
 // run's first slot), then every warp stores whole runs: consecutive lanes,
 // consecutive slots.  No atomics: the run table gives every offset.
-constexpr int STAGE_TILE = bsort::TILE;
+constexpr int STAGE_TILE = bsort::THREADS * kStageIter;
 static_assert(STAGE_TILE == MOVE_CHUNK, "staging tiles are the staging pass's tiles");
 
 __global__ void __launch_bounds__(MOVE_THREADS) stage_scatter_kernel(
@@ -145,7 +150,7 @@ __global__ void __launch_bounds__(MOVE_THREADS) stage_scatter_kernel(
     const double *__restrict__ in, double *__restrict__ out)
 {
     __shared__ double st_val[STAGE_TILE];
-    __shared__ int first[bsort::MAXB], cnt[bsort::MAXB], off[bsort::MAXB];
+    __shared__ int first[kStageBuckets], cnt[kStageBuckets], off[kStageBuckets];
     __shared__ int wsum[MOVE_THREADS / 32];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const long long base = (long long)blockIdx.x * STAGE_TILE;
@@ -196,21 +201,38 @@ __global__ void __launch_bounds__(MOVE_THREADS) stage_scatter_kernel(
     }
 }
 
-// Run table of the staging tiles from the staging pass's scanned digit-major
-// table (pos[b * ntiles + t] = first slot of tile t's entries in bucket b).
-__global__ void stage_runs_kernel(long long nnz, int ntiles, int used, int nb,
-                                  const int *__restrict__ pos, int *__restrict__ run_first,
-                                  unsigned short *__restrict__ run_count)
+// Run table of the staging tiles from the staging pass's tables: the first
+// slot of tile t's entries in bucket b is the bucket's first slot plus the
+// entries of b in earlier chunks and in earlier tiles of the tile's chunk.
+__global__ void __launch_bounds__(kStageBuckets) stage_runs_kernel(
+    int ntiles, int used, int width, int per_chunk, const int *__restrict__ prefix,
+    const int *__restrict__ chunk_base, const int *__restrict__ total,
+    int *__restrict__ run_first, unsigned short *__restrict__ run_count)
 {
-    const long long total = (long long)ntiles * used;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-         i += (long long)gridDim.x * blockDim.x) {
-        const long long t = i / used, b = i - t * used;
-        const long long flat = b * ntiles + t;
-        const long long next = flat + 1 < (long long)nb * ntiles ? __ldg(pos + flat + 1) : nnz;
-        const int f = __ldg(pos + flat);
-        run_first[i] = f;
-        run_count[i] = (unsigned short)(next - f);
+    __shared__ int start[kStageBuckets];
+    const int b = threadIdx.x;
+    const int own = b < width ? __ldg(total + b) : 0;
+    start[b] = own;
+    __syncthreads();
+    for (int k = 1; k < kStageBuckets; k <<= 1) {   // inclusive scan over the buckets
+        const int o = b >= k ? start[b - k] : 0;
+        __syncthreads();
+        start[b] += o;
+        __syncthreads();
+    }
+    const int base = start[b] - own;
+    if (b >= used) return;
+    for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        const long long c = t / per_chunk;
+        const int in_chunk = __ldg(prefix + t * width + b);
+        const int from = __ldg(chunk_base + c * width + b);
+        // the entries of b up to the next tile, inside the chunk or past its end
+        const bool last = t + 1 == ntiles;
+        const int next = last ? own
+                         : (t + 1) % per_chunk ? from + __ldg(prefix + (t + 1) * width + b)
+                                               : __ldg(chunk_base + (c + 1) * width + b);
+        run_first[t * used + b] = base + from + in_chunk;
+        run_count[t * used + b] = (unsigned short)(next - from - in_chunk);
     }
 }
 
@@ -232,25 +254,6 @@ __global__ void __launch_bounds__(MOVE_THREADS) invert_kernel(long long nnz,
         if (t[k] >= 0 && (long long)t[k] < nnz) out[t[k]] = (int)(base + k * MOVE_THREADS);
 }
 
-// The staging pass: CSC entries q keyed by their row position inv[q], one
-// bucket digit (bits and up); the pass writes each entry's staging slot by
-// CSC position (dst) and the row position held by every slot (key_out).
-struct StageOp {
-    const int *key_in;
-    int *key_out;
-    int *a_out = nullptr;
-    int *b_out = nullptr;
-    double *d_out = nullptr;
-    int *pos_out;
-    static constexpr bool kPosOut = true;
-    struct State {};
-    __device__ int key(long long e) const { return __ldg(key_in + e); }
-    __device__ bsort::Payload load(State &, long long, int, bool, long long e) const
-    {
-        return bsort::Payload{0, (int)e, 0.0};
-    }
-};
-
 bool check_work(int m, int n, long long nnz, void *work, size_t work_bytes)
 {
     const size_t need = csc_layout(m, n, nnz).total;
@@ -267,7 +270,7 @@ bool check_work(int m, int n, long long nnz, void *work, size_t work_bytes)
 size_t cscmv_workspace_bytes(int m, int n, long long nnz) { return csc_layout(m, n, nnz).total; }
 
 int launch_csc_analyse(int m, int n, long long nnz, const int *colptr, const int *rowidx,
-                       void *work, size_t work_bytes, bool staged, cudaStream_t stream)
+                       const double *val, void *work, size_t work_bytes, cudaStream_t stream)
 {
     if (m < 0 || n < 0 || nnz < 0 || nnz > 0x7fffffffLL) {
         set_error(SBLAS_ERR_ARG, "bad sizes m=%d n=%d nnz=%lld", m, n, nnz);
@@ -279,16 +282,25 @@ int launch_csc_analyse(int m, int n, long long nnz, const int *colptr, const int
     unsigned char *w = static_cast<unsigned char *>(work);
     int *rowptr = reinterpret_cast<int *>(w + L.rowptr);
     int *perm = reinterpret_cast<int *>(w + L.perm);
+    int rc;
+    if (val != nullptr) {   // one product: the sort carries its values
+        rc = launch_csc_to_csr(m, n, nnz, val, colptr, rowidx,
+                               reinterpret_cast<double *>(w + L.val), rowptr,
+                               reinterpret_cast<int *>(w + L.col), w + L.scratch,
+                               L.total - L.scratch, stream);
+        if (rc != SBLAS_OK) return rc;
+        return launch_tile_analyse(m, nnz, rowptr, kCscSigma, w + L.tile, stream);
+    }
     // the CSC arrays are the CSR arrays of A^T (n rows): its transpose is A
     // in CSR, with every entry's CSC position as the permutation
-    int rc = launch_csr_transpose(n, m, nnz, colptr, rowidx, rowptr,
+    rc = launch_csr_transpose(n, m, nnz, colptr, rowidx, rowptr,
                                   reinterpret_cast<int *>(w + L.col), perm, w + L.scratch,
                                   L.total - L.scratch, stream);
     if (rc != SBLAS_OK) return rc;
     rc = launch_tile_analyse(m, nnz, rowptr, kCscSigma, w + L.tile, stream);
     if (rc != SBLAS_OK) return rc;
     const StagePlan sp = stage_plan(nnz);
-    if (!staged || sp.used <= 1) return SBLAS_OK;
+    if (sp.used <= 1) return SBLAS_OK;
     // staging indices: inv (row position of CSC entry q), the bucket pass
     // giving dst and the row position of every slot, then src (the slot of
     // every row position) in place of perm
@@ -299,18 +311,23 @@ int launch_csc_analyse(int m, int n, long long nnz, const int *colptr, const int
     const unsigned grid = move_grid(nnz);
     invert_kernel<<<grid, MOVE_THREADS, 0, stream>>>(nnz, perm, inv);
     SBLAS_CUDA_TRY(cudaGetLastError());
-    StageOp op;
+    // the staging pass: CSC entries q keyed by their row position inv[q], one
+    // bucket digit (bits and up); it writes each entry's staging slot by CSC
+    // position (dst) and the row position held by every slot
+    bsort::Arrays op;
     op.key_in = inv;
     op.key_out = slot_row;
     op.pos_out = reinterpret_cast<int *>(w + L.dst);
-    rc = bsort::scatter_pass(op, nnz, sp.bits, sp.nb, pass_work, stream);
+    rc = bsort::scatter_pass_iter<false, false, true, kStageIter>(op, nnz, sp.bits, sp.nb,
+                                                                  pass_work, stream);
     if (rc != SBLAS_OK) return rc;
     const long long nt = stage_tiles(nnz);
     const size_t nruns = (size_t)nt * (size_t)sp.used;
-    int *run_first = reinterpret_cast<int *>(w + L.runs);
-    stage_runs_kernel<<<(unsigned)std::min<long long>((nruns + 255) / 256, 8LL * device_num_sms()),
-                        256, 0, stream>>>(
-        nnz, (int)nt, sp.used, sp.nb, static_cast<const int *>(pass_work), run_first,
+    const bsort::PassTables tab = bsort::pass_tables(nnz, sp.nb, kStageIter, pass_work);
+    stage_runs_kernel<<<(unsigned)std::min<long long>(nt, 8LL * device_num_sms()), kStageBuckets,
+                        0, stream>>>(
+        (int)nt, sp.used, bsort::table_width(sp.nb), tab.per_chunk, tab.prefix, tab.chunk_base, tab.total,
+        reinterpret_cast<int *>(w + L.runs),
         reinterpret_cast<unsigned short *>(w + L.runs + al256(4 * nruns)));
     SBLAS_CUDA_TRY(cudaGetLastError());
     invert_kernel<<<grid, MOVE_THREADS, 0, stream>>>(nnz, slot_row, perm);
@@ -319,7 +336,7 @@ int launch_csc_analyse(int m, int n, long long nnz, const int *colptr, const int
 }
 
 int launch_csc_bind_values(int m, int n, long long nnz, const double *val, void *work,
-                           size_t work_bytes, bool staged, cudaStream_t stream)
+                           size_t work_bytes, cudaStream_t stream)
 {
     if (m <= 0 || nnz <= 0) return SBLAS_OK;
     if (!check_work(m, n, nnz, work, work_bytes)) return SBLAS_ERR_ARG;
@@ -329,7 +346,7 @@ int launch_csc_bind_values(int m, int n, long long nnz, const double *val, void 
     double *rval = reinterpret_cast<double *>(w + L.val);
     const unsigned grid = move_grid(nnz);
     const StagePlan sp = stage_plan(nnz);
-    if (staged && sp.used > 1) {
+    if (sp.used > 1) {
         double *stage = reinterpret_cast<double *>(w + L.scratch);
         const size_t nruns = (size_t)stage_tiles(nnz) * (size_t)sp.used;
         stage_scatter_kernel<<<(unsigned)stage_tiles(nnz), MOVE_THREADS, 0, stream>>>(
@@ -347,7 +364,7 @@ int launch_csc_bind_values(int m, int n, long long nnz, const double *val, void 
 
 int launch_cscmv_analysed(int m, int n, long long nnz, double alpha, const double *val,
                           const double *x, double beta, double *y, void *work,
-                          size_t work_bytes, bool staged, cudaStream_t stream)
+                          size_t work_bytes, cudaStream_t stream)
 {
     if (m < 0 || n < 0 || nnz < 0 || nnz > 0x7fffffffLL) {
         set_error(SBLAS_ERR_ARG, "bad sizes m=%d n=%d nnz=%lld", m, n, nnz);
@@ -360,7 +377,7 @@ int launch_cscmv_analysed(int m, int n, long long nnz, double alpha, const doubl
     unsigned char *w = static_cast<unsigned char *>(work);
     double *rval = reinterpret_cast<double *>(w + L.val);
     if (val != nullptr) {   // new values: into row order (else the bound ones)
-        const int rc = launch_csc_bind_values(m, n, nnz, val, work, work_bytes, staged, stream);
+        const int rc = launch_csc_bind_values(m, n, nnz, val, work, work_bytes, stream);
         if (rc != SBLAS_OK) return rc;
     }
     return launch_tile_spmv(m, n, nnz, alpha, rval, VAL_F64,
@@ -373,12 +390,9 @@ int launch_cscmv(int m, int n, long long nnz, double alpha, const double *val,
                  const int *colptr, const int *rowidx, const double *x, double beta, double *y,
                  void *work, size_t work_bytes, cudaStream_t stream)
 {
-    // one product per analysis: the direct gather (staging indices would
-    // cost more to build than they save once)
-    const int rc = launch_csc_analyse(m, n, nnz, colptr, rowidx, work, work_bytes, false, stream);
+    const int rc = launch_csc_analyse(m, n, nnz, colptr, rowidx, val, work, work_bytes, stream);
     if (rc != SBLAS_OK) return rc;
-    return launch_cscmv_analysed(m, n, nnz, alpha, val, x, beta, y, work, work_bytes, false,
-                                 stream);
+    return launch_cscmv_analysed(m, n, nnz, alpha, nullptr, x, beta, y, work, work_bytes, stream);
 }
 
 void *csc_tile_workspace(void *work, int m, int n, long long nnz)

@@ -132,21 +132,21 @@ int launch_csc_to_csr(int m, int n, long long nnz, const double *csc_val,
                       cudaStream_t stream);
 
 // y = alpha*A*x + beta*y with A in CSC (atomic-free, deterministic):
-// inspector (row-ordered structure + permutation + tile partition into
-// `work`) and executor (values into row order + tile kernel).  staged: the
-// inspector also builds the staging indices (an analysis reused for many
-// products) and the executor moves values through them; inspector and
-// executor must agree on it.  work: cscmv_workspace_bytes, 256-byte
-// aligned; csc_tile_workspace: the tile workspace inside it (its status
-// word).
+// inspector (row-ordered structure + tile partition into `work`) and executor
+// (values into row order + tile kernel).  With values, the inspector is the
+// one-shot product's: they are sorted along, and the executor is then called
+// with val = nullptr.  Without, it is an analysis reused for many products:
+// the permutation and the staging indices that the executor moves each
+// product's values through.  work: cscmv_workspace_bytes, 256-byte aligned;
+// csc_tile_workspace: the tile workspace inside it (its status word).
 size_t cscmv_workspace_bytes(int m, int n, long long nnz);
 int launch_csc_analyse(int m, int n, long long nnz, const int *colptr, const int *rowidx,
-                       void *work, size_t work_bytes, bool staged, cudaStream_t stream);
+                       const double *val, void *work, size_t work_bytes, cudaStream_t stream);
 int launch_csc_bind_values(int m, int n, long long nnz, const double *val, void *work,
-                           size_t work_bytes, bool staged, cudaStream_t stream);
+                           size_t work_bytes, cudaStream_t stream);
 int launch_cscmv_analysed(int m, int n, long long nnz, double alpha, const double *val,
                           const double *x, double beta, double *y, void *work,
-                          size_t work_bytes, bool staged, cudaStream_t stream);
+                          size_t work_bytes, cudaStream_t stream);
 int launch_cscmv(int m, int n, long long nnz, double alpha, const double *val,
                  const int *colptr, const int *rowidx, const double *x, double beta, double *y,
                  void *work, size_t work_bytes, cudaStream_t stream);

@@ -114,3 +114,35 @@ def test_spmspv_leaves_out_zero_x(sblas_lib, cuda, kernel, lengths, extra):
         ops.spmspv(trp, long_col, None, tx, y, alpha, beta, kernel=kernel)
         ref = O.csr_spmv(m, n, orp, oc, np.ones(len(oc)), x, y0.copy(), alpha, beta)
         assert rel_l2(y.cpu().numpy(), ref) <= RTOL_L2
+
+
+@pytest.mark.parametrize("nnz", [1, 31, 1023, 1024, 1025, 40_000, (1 << 19) - 1, (1 << 19) + 1,
+                                 (1 << 22) - 1, (1 << 22) + 4097])
+@pytest.mark.parametrize("m,n", [(1, 1), (1, 900), (2, 3_000_000), (2048, 7), (2049, 300),
+                                 (300_000, 1), (5_000_000, 20_000)])
+def test_sorts_at_tile_and_digit_edges(sblas_lib, cuda, nnz, m, n):
+    """CSC -> CSR and the transpose at the edges of the sort's tiles (1024,
+    2048, 4096 entries), digit widths and passes (rows up to 1, 2, 2048, 2049,
+    5M), with few and many, empty and very long columns: whole numbers and
+    values equal to numpy's stable sort."""
+    from hpda_sblas_pnnl_gb300 import ops
+    rng = np.random.default_rng(nnz + m)
+    cols = rng.integers(0, n, nnz)
+    cols[: nnz // 3] = n // 2                      # one long column
+    cols = np.sort(cols)
+    rows = rng.integers(0, m, nnz).astype(np.int32)
+    rows[nnz // 2:] = np.where(rng.random(nnz - nnz // 2) < 0.5, m - 1, rows[nnz // 2:])
+    val = rng.standard_normal(nnz)
+    colptr = np.concatenate([[0], np.cumsum(np.bincount(cols, minlength=n))]).astype(np.int32)
+    order = np.argsort(rows, kind="stable")
+    rowptr = np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=m))])
+    tc, tr, tv = (torch.from_numpy(a).to(cuda) for a in (colptr, rows, val))
+    rp, c, v = ops.csc_to_csr(m, n, tc, tr, tv)
+    assert np.array_equal(rp.cpu().numpy(), rowptr)
+    assert np.array_equal(c.cpu().numpy(), cols[order])
+    assert np.array_equal(v.cpu().numpy(), val[order])
+    # the same arrays as a CSR matrix of n rows: its transpose
+    rp, c, perm = ops.csr_transpose(n, m, tc, tr)
+    assert np.array_equal(rp.cpu().numpy(), rowptr)
+    assert np.array_equal(c.cpu().numpy(), cols[order])
+    assert np.array_equal(perm.cpu().numpy(), order)
