@@ -177,6 +177,7 @@ struct TileArgs {
     const int *row_part;  // [ntiles + 1]
     double *carry;        // [ntiles]
     int *status;          // [1]
+    int clear_status;     // this launch clears it first
     int use_tma;          // val and col 16-byte aligned: bulk copies
     int rp_tma;           // rowptr 16-byte aligned: bulk copies of its tile slices
     int stall;            // test hook: the producer stages nothing, every wait runs out
@@ -243,6 +244,7 @@ struct MultiArgs {
     const int *part;
     double *carry;        // [ntiles], by global tile
     int *status;
+    int clear_status;
     int stall;
     uint64_t wait_ns;
 };
@@ -624,7 +626,7 @@ __device__ __forceinline__ void producer_warp(const Src &src, const Smem<SIGMA, 
         if (t < src.ntiles) {
             const int mat = mat_of(src, t);
             const MatView v = view_of<TILE>(src, t, mat);
-            produce_tile<SIGMA, VK>(v, sm, mat, s, __ldg(v.part), __ldg(v.part + 1), lane,
+            produce_tile<SIGMA, VK>(v, sm, mat, s, v.part[0], v.part[1], lane,
                                     pol_stream);
             ++issued[s];
         }
@@ -634,8 +636,8 @@ __device__ __forceinline__ void producer_warp(const Src &src, const Smem<SIGMA, 
         const int s = i % STAGES;
         const int mat = mat_of(src, nt);
         const MatView v = view_of<TILE>(src, nt, mat);
-        const int R0 = __ldg(v.part);
-        const int R1 = __ldg(v.part + 1);
+        const int R0 = v.part[0];
+        const int R1 = v.part[1];
         const bool ok = ptx::mbar_wait_bounded(sm.empty(s), (uint32_t)((i / STAGES) & 1),
                                                src.wait_ns);
         if (!__all_sync(0xffffffffu, ok)) {
@@ -812,6 +814,7 @@ __global__ void __launch_bounds__(CTA_THREADS, min_ctas<SIGMA, VK>())
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
     const int lane = tid & 31;
+    ptx::griddep_launch_dependents();   // the fix-up's CTAs may wait beside this grid's
     if (tid == 0) {
         for (int s = 0; s < STAGES; ++s) {
             ptx::mbar_init(sm.full(s), 1);
@@ -825,9 +828,14 @@ __global__ void __launch_bounds__(CTA_THREADS, min_ctas<SIGMA, VK>())
     }
     for (int i = tid; i < 2 * L::RCAP; i += CTA_THREADS) sm.rval(0)[i] = 0.0;
     __syncthreads();
-    // launched right behind the tile partition: the set-up above overlapped
-    // its end; nothing in global memory is read before it has finished
+    // launched right behind the tile partition (or the fix-up of the product
+    // before): the set-up above overlapped its end; nothing in global memory is
+    // touched before it has finished
     ptx::griddep_wait();
+    // The status word is cleared here, not by a memset of its own (a launch
+    // and ~1 us per product): a wait of this launch can give up and report at
+    // the earliest one wait limit after its CTA started.
+    if (src.clear_status && blockIdx.x == 0 && tid == 0) *src.status = 0;
     auto roles = [&](const Src &a) {
         if (warp == NCW)
             producer_warp<SIGMA, VK, Src>(a, sm, lane, ptx::policy_evict_first());
@@ -871,18 +879,18 @@ __device__ __forceinline__ void own_tiles(int r, int b, int e, int ntiles, unsig
 
 // Tiles that start at or past rowptr[m] (arrays longer than the row pointer
 // says) own no rows.
-__device__ __forceinline__ void own_no_rows(int m, const int *__restrict__ rowptr, int ntiles,
-                                            unsigned tile, int *__restrict__ part)
+__device__ __forceinline__ void own_no_rows(int m, const int *rowptr, int ntiles,
+                                            unsigned tile, int *part)
 {
     if (blockIdx.x != 0) return;
-    const unsigned end = (unsigned)max(__ldg(rowptr + m), 0);
+    const unsigned end = (unsigned)max(rowptr[m], 0);
     const unsigned long long k0 = ((unsigned long long)end + tile - 1) / tile;
     for (unsigned long long k = max(k0, 1ull) + threadIdx.x; k < (unsigned)ntiles; k += blockDim.x)
         part[k] = m;
 }
 
 __global__ void tile_partition_kernel(int m, long long nnz, int ntiles, long long tile,
-                                      const int *__restrict__ rowptr, int *__restrict__ part)
+                                      const int *rowptr, int *part)
 {
     (void)nnz;
     ptx::griddep_launch_dependents();   // the tile kernel may start its set-up
@@ -894,15 +902,15 @@ __global__ void tile_partition_kernel(int m, long long nnz, int ntiles, long lon
     }
     own_no_rows(m, rowptr, ntiles, (unsigned)tile, part);
     for (int r = g; r < m; r += stride)
-        own_tiles(r, __ldg(rowptr + r), __ldg(rowptr + r + 1), ntiles, (unsigned)tile, part);
+        own_tiles(r, rowptr[r], rowptr[r + 1], ntiles, (unsigned)tile, part);
 }
 
 // The same pass for a 16-byte aligned row pointer: four rows per thread from
 // one 16-byte load (plus the next entry), two such loads in flight; one row
 // per thread kept too few bytes in flight to stream the row pointer.
 __global__ void tile_partition_quad_kernel(int m, int ntiles, long long tile,
-                                           const int *__restrict__ rowptr,
-                                           int *__restrict__ part)
+                                           const int *rowptr,
+                                           int *part)
 {
     ptx::griddep_launch_dependents();   // the tile kernel may start its set-up
     const long long stride = (long long)gridDim.x * blockDim.x;
@@ -924,30 +932,32 @@ __global__ void tile_partition_quad_kernel(int m, int ntiles, long long tile,
     for (long long q = g; q < nq; q += 2 * stride) {
         const long long q2 = q + stride;
         const bool two = q2 < nq;
-        const int4 v = __ldg(q4 + q);
-        const int ve = __ldg(rowptr + 4 * q + 4);
-        const int4 w = two ? __ldg(q4 + q2) : v;
-        const int we = two ? __ldg(rowptr + 4 * q2 + 4) : 0;
+        const int4 v = q4[q];
+        const int ve = rowptr[4 * q + 4];
+        const int4 w = two ? q4[q2] : v;
+        const int we = two ? rowptr[4 * q2 + 4] : 0;
         quad(v, ve, 4 * q);
         if (two) quad(w, we, 4 * q2);
     }
     for (long long r = 4 * nq + g; r < m; r += stride)
-        own_tiles((int)r, __ldg(rowptr + r), __ldg(rowptr + r + 1), ntiles, t32, part);
+        own_tiles((int)r, rowptr[r], rowptr[r + 1], ntiles, t32, part);
 }
 
-// Adds the carries of the tiles a row spans to the row, in tile order.
-__global__ void tile_fixup_kernel(int ntiles, long long tile, double alpha,
-                                  const int *__restrict__ rowptr, const int *__restrict__ part,
-                                  const double *__restrict__ carry, double *__restrict__ y,
-                                  const int *__restrict__ status)
+// Adds the carries of the tiles a row spans to the row, in tile order.  (Plain
+// pointers: what the kernel before wrote is read after griddep_wait, and a
+// load marked as constant could be moved ahead of it.)
+__global__ void tile_fixup_kernel(int ntiles, long long tile, double alpha, const int *rowptr,
+                                  const int *part, const double *carry, double *y,
+                                  const int *status)
 {
+    ptx::griddep_launch_dependents();   // the next product may start its set-up
     ptx::griddep_wait();   // launched behind the tile kernel: its carries are complete
     const int k = blockIdx.x * blockDim.x + threadIdx.x + 1;
     if (k >= ntiles) return;
     if (*status != 0) return;
     const int r = part[k];
     if (part[k + 1] <= r) return;                               // row r ends later
-    if ((long long)__ldg(rowptr + r) >= (long long)k * tile) return;  // starts in tile k
+    if ((long long)rowptr[r] >= (long long)k * tile) return;    // starts in tile k
     int j = k - 1;
     double c = carry[j];
     while (j >= 1 && part[j] == part[j + 1]) {
@@ -967,6 +977,8 @@ __global__ void scale_y_kernel(int m, double beta, double *__restrict__ y)
 // own tiles and partition.
 __global__ void multi_fixup_kernel(const MultiArgs a, long long tile)
 {
+    ptx::griddep_launch_dependents();
+    ptx::griddep_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.ntiles) return;
     if (*a.status != 0) return;
@@ -1169,15 +1181,16 @@ int launch_tile_analyse(int m, long long nnz, const int *rowptr, int sigma, void
     const int ntiles = (int)ntiles_ll;
     int *part = reinterpret_cast<int *>(static_cast<unsigned char *>(work) + kStatusBytes);
     const int threads = 256;
+    // An ordinary launch: as a programmatic dependent of the product before, its
+    // CTAs sat beside that product's and the next tile kernel's CTAs were placed
+    // around them, unevenly over the SMs (power-law step 388 -> 501 us).
     if ((reinterpret_cast<uintptr_t>(rowptr) & 15) == 0) {
         const int quads = m / 4 + 1;
         const int blocks = min((quads + threads - 1) / threads, 8 * device_num_sms());
-        tile_partition_quad_kernel<<<blocks, threads, 0, stream>>>(m, ntiles, tile, rowptr,
-                                                                   part);
+        tile_partition_quad_kernel<<<blocks, threads, 0, stream>>>(m, ntiles, tile, rowptr, part);
     } else {
         const int blocks = min((m + threads - 1) / threads, 8 * device_num_sms());
-        tile_partition_kernel<<<blocks, threads, 0, stream>>>(m, nnz, ntiles, tile, rowptr,
-                                                              part);
+        tile_partition_kernel<<<blocks, threads, 0, stream>>>(m, nnz, ntiles, tile, rowptr, part);
     }
     SBLAS_CUDA_TRY(cudaGetLastError());
     return SBLAS_OK;
@@ -1269,7 +1282,7 @@ int launch_multi_tile_spmv(const MultiTileLaunch &L, int val_kind, cudaStream_t 
     a.status = L.status;
     a.stall = g_stall.load(std::memory_order_relaxed);
     a.wait_ns = g_wait_ns.load(std::memory_order_relaxed);
-    SBLAS_CUDA_TRY(cudaMemsetAsync(L.status, 0, sizeof(int), stream));
+    a.clear_status = 1;
     int rc;
     switch (val_kind) {
     case VAL_F64: rc = launch_shape<11, VAL_F64, 3, MultiArgs>(a, stream); break;
@@ -1282,8 +1295,9 @@ int launch_multi_tile_spmv(const MultiTileLaunch &L, int val_kind, cudaStream_t 
     if (rc != SBLAS_OK) return rc;
     if (a.ntiles > 1) {
         const int threads = 256;
-        multi_fixup_kernel<<<(a.ntiles + threads - 1) / threads, threads, 0, stream>>>(
-            a, (long long)TC * multi_tile_sigma());
+        SBLAS_CUDA_TRY(launch_pdl(multi_fixup_kernel, dim3((a.ntiles + threads - 1) / threads),
+                                  dim3(threads), 0, stream, a,
+                                  (long long)TC * multi_tile_sigma()));
         SBLAS_CUDA_TRY(cudaGetLastError());
     }
     return SBLAS_OK;
@@ -1344,7 +1358,6 @@ int launch_tile_spmv(int m, int n, long long nnz, double alpha, const void *val,
     double *carry = reinterpret_cast<double *>(w + kStatusBytes +
                                                align256(sizeof(int) * (size_t)(ntiles + 1)));
     int *status = status_in(work);
-    if (reset_status) SBLAS_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int), stream));
     if (!analysed) {
         const int rc = launch_tile_analyse(m, nnz, rowptr, sigma, work, stream);
         if (rc != SBLAS_OK) return rc;
@@ -1364,6 +1377,7 @@ int launch_tile_spmv(int m, int n, long long nnz, double alpha, const void *val,
     a.row_part = part;
     a.carry = carry;
     a.status = status;
+    a.clear_status = reset_status ? 1 : 0;
     const uintptr_t vb = reinterpret_cast<uintptr_t>(val), cb = reinterpret_cast<uintptr_t>(col);
     a.use_tma = ((val_kind == VAL_PATTERN || (vb & 15) == 0) && (cb & 15) == 0) ? 1 : 0;
     a.rp_tma = (reinterpret_cast<uintptr_t>(rowptr) & 15) == 0 ? 1 : 0;
