@@ -68,37 +68,39 @@ bool s_compiled(int s) { return s == 4 || s == 8 || s == 16 || s == 32; }
 // units to occupy the 152 SMs; and every unit pays its staging, row search,
 // carries and fix-up, so a large one wants long units, up to where the
 // kernel's shared memory or its lanes' uneven row ends cost more.  Measured
-// (us per product, power-law / banded graphs, CUDA graph of five products):
+// (us per product, power-law / banded graphs of 20 nonzeros per row):
 //            nnz      s = 1         2         4         8        16        32
 //   k = 1   8e3                       7.5/6.3   9.1/6.3  12.4/8.3
 //           2.0e7                     162/164   139/112   166/144   161/132
 //   k = 2   1.6e6                      31/28     26/19     29/22     27/24
-//           4.2e6                      58/62     45/39     42/38     60/63
+//           3.1e6 (6 per row)          64/43     56/32     60/34
+//           2.0e7                     231/275   174/161   168/165   248/262
 //   k = 4   1.6e5                    14.8/10.3 14.0/10.3 15.7/12.8
 //           6.2e5                    23.6/22.6 21.0/18.1 18.1/16.1 22.6/18.5
 //           2.0e7                     380/487   292/297   249/230   335/321
 //   k = 8   8e3     11.1/9.1 12.4/10.3 13.6/12.0 18.1/16.1
 //           1.6e5   22.3/17  17.3/12.8 18.5/12.7 21.0/16.9
-//           6.2e5             37/33     28/27     26/23     38/30
-//           1.6e6             77/78     56/56     49/46     48/40
-//           2.0e7                      548/605   426/455   401/379
+//           6.1e5 (6 per row)          32/28     33/27     48/39
+//           3.1e6 (6 per row)         102/97     90/81    102/89
+//           1.6e7 (80 per row)        436/432   342/342   288/285
+//           2.0e7                     548/605   426/455   401/379
 //   k = 16  8e3     11.6/9.5 14.4/11.5 18.9/15.3 26.3/22.3
 //           1.6e5   25.5/19  19.8/14.0 20.1/15.5 27.1/22.6
-//           6.2e5             43/39     38/37     36/32     50/44
-//           1.6e6             89/95     78/78     72/68     71/64
-//           2.0e7                      785/849   679/723   658/648
+//           6.1e5 (6 per row)          41/37     46/34     66/50
+//           3.1e6 (6 per row)         144/133   139/123   157/138
+//           3.2e6 (80 per row)        137/135   125/121   119/114
+//           2.0e7                     785/849   679/723   658/648
 // FP64 values read through a permutation (a transposed product) stay at 8: a
 // unit's staging waits for random sectors, and more and shorter units hide
 // that better (1M rows, 2.0e7 nonzeros, s = 8 against 16: k = 8 466/471
 // against 577/436 us, k = 16 720/748 against 792/700).
 int pick_s(int k, long long nnz, bool permuted_f64)
 {
-    if (k >= 8 && permuted_f64 && nnz >= 400000) return 8;
     if (k >= 8)
-        return nnz < (1 << 14) ? 1 : nnz < 200000 ? 2 : nnz < 400000 ? 4 : nnz < 1200000 ? 8 : 16;
+        return nnz < (1 << 14) ? 1 : nnz < 200000 ? 2 : nnz < 1000000 ? 4
+               : nnz < 6000000 || permuted_f64 ? 8 : 16;
     if (nnz < (1 << 14)) return 4;
-    if (k == 1) return 8;
-    return nnz < (k == 2 ? 2000000 : 400000) ? 8 : 16;
+    return k == 4 && nnz >= 400000 ? 16 : 8;
 }
 
 bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }

@@ -58,7 +58,7 @@ def test_batch_fixup_run_lengths(sblas_lib, cuda, k):
 
 
 @pytest.mark.parametrize("k", [1, 2, 4, 8, 16])
-@pytest.mark.parametrize("nnz", [3_000, 20_000, 250_000, 500_000, 1_300_000, 2_100_000])
+@pytest.mark.parametrize("nnz", [3_000, 20_000, 250_000, 500_000, 1_300_000, 6_100_000])
 def test_plan_picks_a_shape_for_every_size(sblas_lib, cuda, k, nnz):
     """s = 0 on both sides of each size at which the pick changes, with a
     permuted transpose product: forward and both gradients."""
