@@ -180,9 +180,12 @@ int sblas_dcsrmv(int kernel, int m, int n, long long nnz, double alpha, const vo
             set_error(SBLAS_ERR_UNSUPPORTED, "kernel 1 takes FP64 values only");
             return SBLAS_ERR_UNSUPPORTED;
         }
+        if (nnz > 0 && small_spmv_fits(m, n, nnz, false))
+            return launch_small_spmv(m, alpha, val, val_kind, rowptr, col, x, beta, y, nullptr, st);
         return launch_rowsplit_spmv(m, n, nnz, alpha, static_cast<const double *>(val), rowptr,
                                     col, x, beta, y, st);
     }
+    const bool auto_shape = sigma <= 0;
     if (sigma <= 0)
         sigma = (kernel == SBLAS_KERNEL_CSR5) ? csr5_sigma_for(m, nnz) : default_sigma_for(m, nnz);
     const size_t need = tile_workspace_bytes(nnz, sigma);
@@ -197,7 +200,7 @@ int sblas_dcsrmv(int kernel, int m, int n, long long nnz, double alpha, const vo
         return SBLAS_ERR_ARG;
     }
     return launch_tile_spmv(m, n, nnz, alpha, val, val_kind, rowptr, col, x, beta, y, sigma,
-                            work, st);
+                            work, st, false, true, false, auto_shape);
 }
 
 int sblas_csr_analyse(int kernel, int m, long long nnz, const int *rowptr, int sigma, void *work,
@@ -236,6 +239,7 @@ int sblas_dcsrmv_analysed(int kernel, int m, int n, long long nnz, double alpha,
         set_error(SBLAS_ERR_ARG, "null device pointer");
         return SBLAS_ERR_ARG;
     }
+    const bool auto_shape = sigma <= 0;
     if (sigma <= 0)
         sigma = (kernel == SBLAS_KERNEL_CSR5) ? csr5_sigma_for(m, nnz) : default_sigma_for(m, nnz);
     if (work_bytes < tile_workspace_bytes(nnz, sigma) ||
@@ -245,7 +249,7 @@ int sblas_dcsrmv_analysed(int kernel, int m, int n, long long nnz, double alpha,
         return SBLAS_ERR_ARG;
     }
     return launch_tile_spmv(m, n, nnz, alpha, val, val_kind, rowptr, col, x, beta, y, sigma, work,
-                            static_cast<cudaStream_t>(stream), true);
+                            static_cast<cudaStream_t>(stream), true, true, false, auto_shape);
 }
 
 int sblas_dcoomv(int m, int n, long long nnz, double alpha, const double *val,
@@ -423,6 +427,9 @@ int sblas_dspmspv(int kernel, int m, int n, long long nnz, double alpha, const d
             set_error(SBLAS_ERR_UNSUPPORTED, "kernel 1 takes FP64 values only");
             return SBLAS_ERR_UNSUPPORTED;
         }
+        if (nnz > 0 && small_spmv_fits(m, n, nnz, false))
+            return launch_small_spmv(m, alpha, val, VAL_F64, rowptr, col, x, beta, y, nullptr, st,
+                                     true);
         return launch_rowsplit_spmv(m, n, nnz, alpha, val, rowptr, col, x, beta, y, st, true);
     }
     const int sigma = default_sigma_for(m, nnz);
@@ -433,7 +440,7 @@ int sblas_dspmspv(int kernel, int m, int n, long long nnz, double alpha, const d
         return SBLAS_ERR_ARG;
     }
     return launch_tile_spmv(m, n, nnz, alpha, val, val ? VAL_F64 : VAL_PATTERN, rowptr, col, x,
-                            beta, y, sigma, work, st, false, true, true);
+                            beta, y, sigma, work, st, false, true, true, true);
 }
 
 int sblas_zero(void *p, size_t bytes, void *stream)

@@ -364,7 +364,8 @@ spmv_ret run_host(Call c)
                 return failed();
             }
             rc = launch_tile_spmv(rows, n, nnz, c.alpha, val, SBLAS_VAL_F64, rp, col, d_x,
-                                  beta_eff, yp, tile_sigma, tile_work, st);
+                                  beta_eff, yp, tile_sigma, tile_work, st, false, true, false,
+                                  true);
         }
         if (rc != SBLAS_OK) return failed();
     }

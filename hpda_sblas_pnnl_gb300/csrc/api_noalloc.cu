@@ -115,7 +115,7 @@ int sblas_dcsrmv_noalloc(int m, int n, int nnz, double alpha, const double *val,
         return SBLAS_ERR_ARG;
     }
     return launch_tile_spmv(m, n, nnz, alpha, val, SBLAS_VAL_F64, rowptr, col, x, beta, y, sigma,
-                            scratch, static_cast<cudaStream_t>(stream));
+                            scratch, static_cast<cudaStream_t>(stream), false, true, false, true);
 }
 
 }  // extern "C"

@@ -383,7 +383,7 @@ int launch_cscmv_analysed(int m, int n, long long nnz, double alpha, const doubl
     return launch_tile_spmv(m, n, nnz, alpha, rval, VAL_F64,
                             reinterpret_cast<const int *>(w + L.rowptr),
                             reinterpret_cast<const int *>(w + L.col), x, beta, y, kCscSigma,
-                            w + L.tile, stream, true);
+                            w + L.tile, stream, true, true, false, true);
 }
 
 int launch_cscmv(int m, int n, long long nnz, double alpha, const double *val,

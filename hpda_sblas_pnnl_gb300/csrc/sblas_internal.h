@@ -52,6 +52,7 @@ enum ValueKind { VAL_F64 = 0, VAL_F32 = 1, VAL_PATTERN = 2 };
 // `work` must hold tile_workspace_bytes(nnz, sigma) bytes, 256-byte aligned.
 // analysed = true: the partition of `work` was computed by
 // launch_tile_analyse for this row pointer and sigma (skipped here).
+// auto_shape: the caller gave no shape (small matrices then need no tiles).
 // skip_zero_x: nonzeros whose x entry is zero are left out (spMspV), and col
 // and val may be longer than rowptr[m]; sigma 11, FP64 or pattern-only.
 // reset_status = false keeps the workspace's status word as it is (a call
@@ -59,7 +60,8 @@ enum ValueKind { VAL_F64 = 0, VAL_F32 = 1, VAL_PATTERN = 2 };
 int launch_tile_spmv(int m, int n, long long nnz, double alpha, const void *val,
                      int val_kind, const int *rowptr, const int *col, const double *x,
                      double beta, double *y, int sigma, void *work, cudaStream_t stream,
-                     bool analysed = false, bool reset_status = true, bool skip_zero_x = false);
+                     bool analysed = false, bool reset_status = true, bool skip_zero_x = false,
+                     bool auto_shape = false);
 // Status word of a tile workspace (0 = every wait completed), read with a
 // synchronous copy: the caller has synchronised the launches' stream.
 int tile_workspace_status(void *work, int *out);
@@ -99,6 +101,15 @@ void set_wait_limit_ns(unsigned long long ns);
 void set_test_stall(int on);
 int launch_tile_analyse(int m, long long nnz, const int *rowptr, int sigma, void *work,
                         cudaStream_t stream);
+
+// Small matrices (spmv_small.cu): one launch, no workspace.  Callers that
+// leave the tile shape to the library take it where small_spmv_fits.
+// status: cleared, or null.  skip_zero_x as in launch_tile_spmv.
+bool small_spmv_fits(int m, int n, long long nnz, bool analysed);
+int launch_small_spmv(int m, double alpha, const void *val, int val_kind, const int *rowptr,
+                      const int *col, const double *x, double beta, double *y, int *status,
+                      cudaStream_t stream, bool skip_zero_x = false);
+int small_spmv_preload_f64();
 
 // Row-split kernel (one sub-warp per row; kernel version 1).
 int launch_rowsplit_spmv(int m, int n, long long nnz, double alpha, const double *val,

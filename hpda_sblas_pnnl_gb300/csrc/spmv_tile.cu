@@ -1244,6 +1244,7 @@ int tile_preload_f64(int sigma)
         set_error(SBLAS_ERR_UNSUPPORTED, "sigma %d is not a compiled tile shape", sigma);
         return SBLAS_ERR_UNSUPPORTED;
     }
+    if (rc == SBLAS_OK) rc = small_spmv_preload_f64();
     if (rc != SBLAS_OK) return rc;
     cudaFuncAttributes fa;
     SBLAS_CUDA_TRY(cudaFuncGetAttributes(&fa, tile_partition_kernel));
@@ -1338,10 +1339,13 @@ void set_test_stall(int on) { g_stall.store(on ? 1 : 0, std::memory_order_relaxe
 int launch_tile_spmv(int m, int n, long long nnz, double alpha, const void *val, int val_kind,
                      const int *rowptr, const int *col, const double *x, double beta, double *y,
                      int sigma, void *work, cudaStream_t stream, bool analysed, bool reset_status,
-                     bool skip_zero_x)
+                     bool skip_zero_x, bool auto_shape)
 {
     if (m <= 0) return SBLAS_OK;
     if (nnz <= 0) return launch_scale_y(m, beta, y, stream);
+    if (auto_shape && small_spmv_fits(m, n, nnz, analysed))
+        return launch_small_spmv(m, alpha, val, val_kind, rowptr, col, x, beta, y,
+                                 reset_status ? status_in(work) : nullptr, stream, skip_zero_x);
     if (tile_shape_index(sigma) < 0) {
         set_error(SBLAS_ERR_UNSUPPORTED, "sigma %d is not a compiled tile shape", sigma);
         return SBLAS_ERR_UNSUPPORTED;

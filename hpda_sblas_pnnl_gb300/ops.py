@@ -261,6 +261,8 @@ class CsrPlan:
         self.nnz = col.numel()
         self.n = int(n) if n is not None else None
         self.kernel = kernel
+        # 0: the library picks, and runs small matrices without tiles
+        self._sigma = max(int(sigma), 0)
         if sigma <= 0:
             sigma = (lib.sblas_csr5_sigma(self.m, self.nnz) if kernel == KERNEL_CSR5
                      else lib.sblas_default_sigma(self.m, self.nnz))
@@ -293,7 +295,7 @@ class CsrPlan:
         lib = _lib.load()
         rc = lib.sblas_dcsrmv_analysed(self.kernel, self.m, n, self.nnz, float(alpha),
                                        _ptr(self.val), self.vk, _ptr(self.rowptr), _ptr(self.col),
-                                       _ptr(x), float(beta), _ptr(y), self.sigma, _ptr(self.work),
+                                       _ptr(x), float(beta), _ptr(y), self._sigma, _ptr(self.work),
                                        self.work_bytes, _stream_ptr(self.device))
         _lib.check(rc)
         return y

@@ -146,3 +146,38 @@ def test_sorts_at_tile_and_digit_edges(sblas_lib, cuda, nnz, m, n):
     assert np.array_equal(rp.cpu().numpy(), rowptr)
     assert np.array_equal(c.cpu().numpy(), cols[order])
     assert np.array_equal(perm.cpu().numpy(), order)
+
+
+@pytest.mark.parametrize("lengths", [[1], [0, 64, 65, 0, 512, 513], [8192], [8193], [0] * 3000 + [5],
+                                     [7, 0, 63, 64, 65, 511, 512, 513, 4097, 1] * 7,
+                                     [2] * 16_384, [2] * 16_385, [9] * 3641, [9] * 14_563,
+                                     [5, 0, 700, 3] * 40], ids=lambda v: f"{len(v)}x{max(v)}")
+def test_small_matrices(sblas_lib, cuda, lengths):
+    """Rows at the lengths where lanes, warps and the CTA change over, sizes on
+    both sides of the small path's limits, every value kind, alpha and beta,
+    kernels 1 to 3, per call and analysed, an explicit tile shape, x zeros
+    left out, NaN in y with beta = 0."""
+    from hpda_sblas_pnnl_gb300 import ops
+    n = 3000
+    (rp, col, val), (trp, tcol, tval) = csr_of_lengths(lengths, n, 3, cuda)
+    m = len(lengths)
+    rng = np.random.default_rng(m)
+    x = rng.standard_normal(n)
+    tx = torch.from_numpy(x).to(cuda)
+    y0 = rng.standard_normal(m)
+    vals = {"f64": (tval, val), "f32": (tval.float(), tval.float().double().cpu().numpy()),
+            "pattern": (None, np.ones(len(val)))}
+    for form, (tv, v) in vals.items():
+        plan = ops.CsrPlan(trp, tcol, tv, n=n)
+        for alpha, beta in ((1.0, 0.0), (1.5, 0.0), (1.5, -0.5)):
+            start = np.full(m, np.nan) if beta == 0.0 else y0
+            ref = O.csr_spmv(m, n, rp, col, v, x, np.where(np.isnan(start), 0.0, start), alpha, beta)
+            got = {}
+            for kernel in (1, 2, 3) if form == "f64" else (2, 3):
+                y = torch.from_numpy(start).to(cuda)
+                got[f"kernel {kernel}"] = ops.csrmv(trp, tcol, tv, tx, y, alpha, beta, kernel=kernel)
+            got["plan"] = plan(tx, torch.from_numpy(start).to(cuda), alpha, beta)
+            got["sigma"] = ops.csrmv(trp, tcol, tv, tx, torch.from_numpy(start).to(cuda), alpha,
+                                     beta, sigma=15)
+            for what, y in got.items():
+                assert rel_l2(y.cpu().numpy(), ref) <= RTOL_L2, (form, what, alpha, beta)
