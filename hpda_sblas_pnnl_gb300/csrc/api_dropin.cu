@@ -131,22 +131,14 @@ bool check_kernel(const char *name, int kernel)
     return true;
 }
 
-// Row pointer of one chunk rebased to its first nonzero: out[i] = rp[i] - base.
-__global__ void rebase_rowptr_kernel(int count, const int *__restrict__ rp, int base, int *out)
-{
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
-        out[i] = rp[i] - base;
-}
-
 constexpr long long kPipeMinNnz = 1LL << 22;   // smaller matrices: copy, then compute
 
 // After the call's stream has completed: false (with SBLAS_ERR_TIMEOUT set)
-// if a tile launch on workspace w gave up one of its bounded waits, which
-// leaves y partly written.
-bool launches_completed(const Call &c, void *w)
+// if a tile launch of the call gave up one of its bounded waits (the status
+// word, copied to the context's pinned word), which leaves y partly written.
+bool launches_completed(const Call &c, const DeviceContext *ctx)
 {
-    int word = 0;
-    if (tile_workspace_status(w, &word) != SBLAS_OK) return false;
+    const int word = *ctx->host_word;
     if (word != 0) {
         set_error(SBLAS_ERR_TIMEOUT, "%s: the SpMV kernel gave up a bounded wait (device word "
                   "%d); y is not valid", c.name, word);
@@ -155,14 +147,28 @@ bool launches_completed(const Call &c, void *w)
     return true;
 }
 
-// Large CSR calls with host arrays: the matrix travels in kPipeChunks row
-// chunks of equal nonzero counts, each chunk's SpMV starting as soon as its
-// values and columns have arrived (copies on the context's copy stream, the
-// tile kernel on its compute stream, y of a chunk sent back right after its
-// kernel), so the kernels and the device-to-host copies hide behind the
-// host-to-device copies, which the host link bounds.  Each chunk's arrays
-// are placed at 256-byte aligned offsets so the tile kernel keeps its bulk
-// copies; its row pointer is rebased to the chunk's first nonzero.
+// Whether copies to this host memory are asynchronous (pinned): a copy to or
+// from pageable memory returns when it has been done.
+bool is_pinned(const void *p)
+{
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeHost;
+}
+
+// Large CSR calls with host arrays: the matrix travels in kPipeChunks chunks of
+// whole tiles, and the tiles of a chunk run as soon as its values and columns
+// have arrived (copies on the context's copy stream, kernels on its compute
+// stream), so the kernels hide behind the host-to-device copies, which the host
+// link bounds.  A copy from pageable memory blocks the host until it is done:
+// each chunk's kernels are therefore launched before the next chunk's copies
+// are issued (all copies first: no kernel started before the last byte had
+// arrived, 820 us per call with 7.7M nonzeros).  One partition serves all
+// chunks; they share the row pointer as it is.  y goes back chunk by chunk from
+// pinned memory, in one copy at the end to pageable memory.
 spmv_ret run_host_pipelined(const Call &c, DeviceContext *ctx)
 {
     const int m = c.m, n = c.n;
@@ -170,99 +176,71 @@ spmv_ret run_host_pipelined(const Call &c, DeviceContext *ctx)
     const int K = kPipeChunks;
     const bool need_y_in = (c.beta != 0.0) || c.additive;
     cudaStream_t cs = ctx->copy_stream, ks = ctx->stream;
-    // chunk k: rows [r[k], r[k+1]), nonzeros [ptr[r[k]], ptr[r[k+1]])
-    int r[kPipeChunks + 1];
-    r[0] = 0;
-    r[K] = m;
-    for (int k = 1; k < K; ++k) {
-        const long long want = nnz * k / K;
-        int lo = r[k - 1], hi = m;   // first row with ptr[row] >= want
-        while (lo < hi) {
-            const int mid = lo + (hi - lo) / 2;
-            if (c.ptr[mid] >= want) hi = mid; else lo = mid + 1;
-        }
-        r[k] = lo;
-    }
-    const size_t pad = 256;
-    double *d_val = static_cast<double *>(device_scratch(1, sizeof(double) * (size_t)nnz + K * pad));
-    int *d_idx = static_cast<int *>(device_scratch(2, sizeof(int) * (size_t)nnz + K * pad));
+    const int sigma = (c.kernel == 3) ? csr5_sigma_for(m, nnz) : default_sigma_for(m, nnz);
+    const int ntiles = tile_count(nnz, sigma);
+    const long long tile = (long long)tile_shape_at(0).threads * sigma;
+    double *d_val = static_cast<double *>(device_scratch(1, sizeof(double) * (size_t)nnz));
+    int *d_idx = static_cast<int *>(device_scratch(2, sizeof(int) * (size_t)nnz));
     int *d_ptr = static_cast<int *>(device_scratch(3, sizeof(int) * (size_t)(m + 1)));
     double *d_x = static_cast<double *>(device_scratch(4, sizeof(double) * (size_t)n));
     double *d_y = static_cast<double *>(device_scratch(5, sizeof(double) * (size_t)m));
-    int *d_rp = static_cast<int *>(device_scratch(8, sizeof(int) * (size_t)(m + 1 + K) + K * pad));
-    const int sigma = (c.kernel == 3) ? csr5_sigma_for(m, nnz) : default_sigma_for(m, nnz);
     void *w = device_scratch(0, tile_workspace_bytes(nnz, sigma));
-    if (!d_val || !d_idx || !d_ptr || !d_x || !d_y || !d_rp || !w) {
+    if (!d_val || !d_idx || !d_ptr || !d_x || !d_y || !w) {
         set_error(SBLAS_ERR_ALLOC, "%s: device allocation failed", c.name);
         return failed();
     }
-    auto up = [](size_t b) { return (b + 255) & ~size_t(255); };
     cudaEvent_t e0 = ctx->ev[0], e1 = ctx->ev[1], e2 = ctx->ev[2], e3 = ctx->ev[3];
-    // ---- inputs every chunk needs: row pointer, x (and y when it is read)
+    const bool y_pinned = is_pinned(c.y);
+    // ---- the row pointer and its partition, then x (and y when it is read)
     DROPIN_CUDA(cudaEventRecord(e0, cs));
     DROPIN_CUDA(cudaMemcpyAsync(d_ptr, c.ptr, sizeof(int) * (size_t)(m + 1), cudaMemcpyHostToDevice, cs));
+    DROPIN_CUDA(cudaEventRecord(ctx->chunk_ev[0], cs));
+    DROPIN_CUDA(cudaStreamWaitEvent(ks, ctx->chunk_ev[0], 0));
+    DROPIN_CUDA(cudaEventRecord(e2, ks));
+    if (launch_tile_analyse(m, nnz, d_ptr, sigma, w, ks) != SBLAS_OK) return failed();
     DROPIN_CUDA(cudaMemcpyAsync(d_x, c.x, sizeof(double) * (size_t)n, cudaMemcpyHostToDevice, cs));
     if (need_y_in)
         DROPIN_CUDA(cudaMemcpyAsync(d_y, c.y, sizeof(double) * (size_t)m, cudaMemcpyHostToDevice, cs));
-    DROPIN_CUDA(cudaEventRecord(ctx->chunk_ev[0], cs));
-    // ---- the chunks' values and columns
-    size_t vo[kPipeChunks], io[kPipeChunks], ro[kPipeChunks];
-    size_t voff = 0, ioff = 0, roff = 0;
-    for (int k = 0; k < K; ++k) {
-        const long long lo = c.ptr[r[k]], hi = c.ptr[r[k + 1]];
-        vo[k] = voff;
-        io[k] = ioff;
-        ro[k] = roff;
-        if (hi > lo) {
-            DROPIN_CUDA(cudaMemcpyAsync(reinterpret_cast<unsigned char *>(d_val) + voff, c.val + lo,
-                                        sizeof(double) * (size_t)(hi - lo), cudaMemcpyHostToDevice, cs));
-            DROPIN_CUDA(cudaMemcpyAsync(reinterpret_cast<unsigned char *>(d_idx) + ioff, c.idx + lo,
-                                        sizeof(int) * (size_t)(hi - lo), cudaMemcpyHostToDevice, cs));
-        }
-        DROPIN_CUDA(cudaEventRecord(ctx->chunk_ev[1 + k], cs));
-        voff += up(sizeof(double) * (size_t)(hi - lo));
-        ioff += up(sizeof(int) * (size_t)(hi - lo));
-        roff += up(sizeof(int) * (size_t)(r[k + 1] - r[k] + 1));
-    }
-    DROPIN_CUDA(cudaEventRecord(e1, cs));
-    // ---- per chunk: rebase its row pointer, SpMV, send its rows of y back
-    DROPIN_CUDA(cudaStreamWaitEvent(ks, ctx->chunk_ev[0], 0));
-    DROPIN_CUDA(cudaEventRecord(e2, ks));
+    // ---- the chunks: copies, then their tiles
     const double beta_eff = c.additive ? c.beta + 1.0 : c.beta;
-    bool status_cleared = false;
+    int row = 0;
     for (int k = 0; k < K; ++k) {
-        const int rows = r[k + 1] - r[k];
-        if (rows == 0) continue;
-        const long long lo = c.ptr[r[k]], cnnz = c.ptr[r[k + 1]] - lo;
-        int *rp = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(d_rp) + ro[k]);
-        rebase_rowptr_kernel<<<(rows + 1 + 255) / 256 < 1024 ? (rows + 1 + 255) / 256 : 1024, 256, 0, ks>>>(
-            rows + 1, d_ptr + r[k], (int)lo, rp);
-        DROPIN_CUDA(cudaGetLastError());
+        const int t0 = (int)((long long)ntiles * k / K), t1 = (int)((long long)ntiles * (k + 1) / K);
+        if (t1 == t0) continue;
+        const long long lo = t0 * tile, hi = t1 == ntiles ? nnz : t1 * tile;
+        DROPIN_CUDA(cudaMemcpyAsync(d_val + lo, c.val + lo, sizeof(double) * (size_t)(hi - lo),
+                                    cudaMemcpyHostToDevice, cs));
+        DROPIN_CUDA(cudaMemcpyAsync(d_idx + lo, c.idx + lo, sizeof(int) * (size_t)(hi - lo),
+                                    cudaMemcpyHostToDevice, cs));
+        DROPIN_CUDA(cudaEventRecord(ctx->chunk_ev[1 + k], cs));
+        if (t1 == ntiles) DROPIN_CUDA(cudaEventRecord(e1, cs));
         DROPIN_CUDA(cudaStreamWaitEvent(ks, ctx->chunk_ev[1 + k], 0));
-        const double *val = reinterpret_cast<const double *>(reinterpret_cast<unsigned char *>(d_val) + vo[k]);
-        const int *col = reinterpret_cast<const int *>(reinterpret_cast<unsigned char *>(d_idx) + io[k]);
-        // the chunks share one workspace: its status word is cleared once,
-        // by the first launch, so a chunk that gave up a wait stays visible
-        const int rc = (cnnz == 0)
-                           ? launch_scale_y(rows, beta_eff, d_y + r[k], ks)
-                           : launch_tile_spmv(rows, n, cnnz, c.alpha, val, SBLAS_VAL_F64, rp, col, d_x,
-                                              beta_eff, d_y + r[k], sigma, w, ks, false,
-                                              !status_cleared);
-        if (cnnz > 0) status_cleared = true;
-        if (rc != SBLAS_OK) return failed();
-        DROPIN_CUDA(cudaMemcpyAsync(c.y + r[k], d_y + r[k], sizeof(double) * (size_t)rows,
-                                    cudaMemcpyDeviceToHost, ks));
+        if (launch_tile_range(m, n, nnz, c.alpha, d_val, SBLAS_VAL_F64, d_ptr, d_idx, d_x, beta_eff,
+                              d_y, sigma, w, ks, t0, t1, t0 == 0) != SBLAS_OK)
+            return failed();
+        if (!y_pinned) continue;
+        // the rows that end before tile t1 are complete
+        const int end = t1 == ntiles ? m
+                                     : (int)(std::upper_bound(c.ptr + 1, c.ptr + m + 1, (int)hi) -
+                                             (c.ptr + 1));
+        if (end > row)
+            DROPIN_CUDA(cudaMemcpyAsync(c.y + row, d_y + row, sizeof(double) * (size_t)(end - row),
+                                        cudaMemcpyDeviceToHost, ks));
+        row = std::max(row, end);
     }
+    if (tile_workspace_status(w, ctx->host_word, ks) != SBLAS_OK) return failed();
     DROPIN_CUDA(cudaEventRecord(e3, ks));
     const double tm = wall();
-    DROPIN_CUDA(cudaEventSynchronize(e3));
-    if (!launches_completed(c, w)) return failed();
+    if (!y_pinned)
+        DROPIN_CUDA(cudaMemcpyAsync(c.y, d_y, sizeof(double) * (size_t)m, cudaMemcpyDeviceToHost, ks));
+    DROPIN_CUDA(cudaStreamSynchronize(ks));
+    if (!launches_completed(c, ctx)) return failed();
     spmv_ret ret = zero_ret();
     float t_comm = 0.f, t_comp = 0.f;
     DROPIN_CUDA(cudaEventElapsedTime(&t_comm, e0, e1));
     DROPIN_CUDA(cudaEventElapsedTime(&t_comp, e2, e3));
     ret.comm_time = t_comm * 1e-3;   // host-to-device copies (overlapping the kernels)
-    ret.comp_time = t_comp * 1e-3;   // kernels and the copies of y back, from the first chunk on
+    ret.comp_time = t_comp * 1e-3;   // kernels (and copies of y back) from the partition on
     ret.merg_time = wall() - tm;
     return ret;
 }
@@ -298,6 +276,7 @@ spmv_ret run_host(Call c)
         return failed();
     }
     cudaEvent_t e0 = ctx->ev[0], e1 = ctx->ev[1], e2 = ctx->ev[2], e3 = ctx->ev[3];
+    cudaEvent_t e4 = ctx->ev[4];
     // ---- host -> device
     DROPIN_CUDA(cudaEventRecord(e0, st));
     if (nnz > 0) {
@@ -370,20 +349,24 @@ spmv_ret run_host(Call c)
         if (rc != SBLAS_OK) return failed();
     }
     DROPIN_CUDA(cudaEventRecord(e3, st));
-    DROPIN_CUDA(cudaEventSynchronize(e3));
-    if (tile_work && !launches_completed(c, tile_work)) return failed();
-    float t_comm = 0.f, t_part = 0.f, t_comp = 0.f;
-    DROPIN_CUDA(cudaEventElapsedTime(&t_comm, e0, e1));
-    DROPIN_CUDA(cudaEventElapsedTime(&t_part, e1, e2));
-    DROPIN_CUDA(cudaEventElapsedTime(&t_comp, e2, e3));
 
-    // ---- device -> host: only the rows this call writes
-    const double tm = wall();
+    // ---- device -> host: only the rows this call writes, and the tile
+    // launch's status word
+    *ctx->host_word = 0;
+    if (tile_work && tile_workspace_status(tile_work, ctx->host_word, st) != SBLAS_OK)
+        return failed();
     if (rows > 0)
         DROPIN_CUDA(cudaMemcpyAsync(c.y + c.row_lo, d_y + c.row_lo, sizeof(double) * rows,
                                     cudaMemcpyDeviceToHost, st));
+    DROPIN_CUDA(cudaEventRecord(e4, st));
     DROPIN_CUDA(cudaStreamSynchronize(st));
-    ret.merg_time = wall() - tm;
+    if (!launches_completed(c, ctx)) return failed();
+    float t_comm = 0.f, t_part = 0.f, t_comp = 0.f, t_merg = 0.f;
+    DROPIN_CUDA(cudaEventElapsedTime(&t_comm, e0, e1));
+    DROPIN_CUDA(cudaEventElapsedTime(&t_part, e1, e2));
+    DROPIN_CUDA(cudaEventElapsedTime(&t_comp, e2, e3));
+    DROPIN_CUDA(cudaEventElapsedTime(&t_merg, e3, e4));
+    ret.merg_time = t_merg * 1e-3;
     ret.comm_time = t_comm * 1e-3;
     ret.part_time = t_part * 1e-3;
     ret.comp_time = t_comp * 1e-3;

@@ -62,9 +62,18 @@ int launch_tile_spmv(int m, int n, long long nnz, double alpha, const void *val,
                      double beta, double *y, int sigma, void *work, cudaStream_t stream,
                      bool analysed = false, bool reset_status = true, bool skip_zero_x = false,
                      bool auto_shape = false);
-// Status word of a tile workspace (0 = every wait completed), read with a
-// synchronous copy: the caller has synchronised the launches' stream.
-int tile_workspace_status(void *work, int *out);
+// Tiles [t0, t1) of the product (and the fix-up of the rows that end in them)
+// after launch_tile_analyse on the same workspace: a caller that receives the
+// matrix in pieces runs each as it arrives, in order.  tile_count: the tiles of
+// 128 * sigma nonzeros.
+int tile_count(long long nnz, int sigma);
+int launch_tile_range(int m, int n, long long nnz, double alpha, const void *val, int val_kind,
+                      const int *rowptr, const int *col, const double *x, double beta, double *y,
+                      int sigma, void *work, cudaStream_t stream, int t0, int t1,
+                      bool reset_status, bool skip_zero_x = false);
+// Status word of a tile workspace (0 = every wait completed), copied to *out
+// (host memory that stays until the stream has completed) in stream order.
+int tile_workspace_status(void *work, int *out, cudaStream_t stream);
 // The sticky per-device word (any tile launch that gave up a wait), read
 // after `stream` completes; clear = reset it to 0.
 int tile_sticky_status(cudaStream_t stream, bool clear, int *out);
@@ -181,7 +190,8 @@ struct DeviceContext {
     cudaStream_t stream = nullptr;
     cudaStream_t copy_stream = nullptr;   // host -> device copies overlapping the kernels
     cudaEvent_t ev[6] = {};
-    cudaEvent_t chunk_ev[kPipeChunks + 1] = {};  // copies done (inputs, then each chunk)
+    cudaEvent_t chunk_ev[kPipeChunks + 2] = {};  // copies done (row pointer, x and y, each chunk)
+    int *host_word = nullptr;   // pinned: a launch's status word
 };
 // Returns the context of the current device (created on first use).
 DeviceContext *device_context();

@@ -166,6 +166,7 @@ struct TileArgs {
     int m;
     int n;
     long long nnz;
+    int tile0;            // tiles [tile0, ntiles) of the matrix run in this launch
     int ntiles;
     double alpha;
     double beta;
@@ -207,6 +208,7 @@ struct MatView {
 // Source of tiles: one matrix (TileArgs) or many (MultiArgs, below).  Both
 // give the total tile count, a tile's matrix and the tile's view of it.
 __device__ __forceinline__ int mat_of(const TileArgs &, int) { return 0; }
+__host__ __device__ __forceinline__ int first_tile(const TileArgs &a) { return a.tile0; }
 
 template <int TILE>
 __device__ __forceinline__ MatView view_of(const TileArgs &a, int tile, int)
@@ -248,6 +250,8 @@ struct MultiArgs {
     int stall;
     uint64_t wait_ns;
 };
+
+__host__ __device__ __forceinline__ int first_tile(const MultiArgs &) { return 0; }
 
 __device__ __forceinline__ int mat_of(const MultiArgs &a, int tile)
 {
@@ -429,7 +433,8 @@ __device__ __forceinline__ void compute_warp(const Src &src, const Smem<SIGMA, V
     using VT = typename ValTraits<VK>::T;
     constexpr int TILE = L::TILE;
     const int t = cw * 32 + lane;
-    for (int i = 0, tile = blockIdx.x; tile < src.ntiles; ++i, tile += gridDim.x) {
+    for (int i = 0, tile = first_tile(src) + blockIdx.x; tile < src.ntiles;
+         ++i, tile += gridDim.x) {
         const int s = i % STAGES;
         const int p = i & 1;
         bool ok = ptx::mbar_wait_bounded(sm.full(s), (uint32_t)((i / STAGES) & 1), src.wait_ns);
@@ -622,7 +627,7 @@ __device__ __forceinline__ void producer_warp(const Src &src, const Smem<SIGMA, 
 #pragma unroll
     for (int s = 0; s < STAGES; ++s) issued[s] = 0;
     for (int s = 0; s < STAGES; ++s) {
-        const int t = blockIdx.x + s * (int)gridDim.x;
+        const int t = first_tile(src) + blockIdx.x + s * (int)gridDim.x;
         if (t < src.ntiles) {
             const int mat = mat_of(src, t);
             const MatView v = view_of<TILE>(src, t, mat);
@@ -631,7 +636,7 @@ __device__ __forceinline__ void producer_warp(const Src &src, const Smem<SIGMA, 
             ++issued[s];
         }
     }
-    for (int i = 0, nt = blockIdx.x + STAGES * (int)gridDim.x; nt < src.ntiles;
+    for (int i = 0, nt = first_tile(src) + blockIdx.x + STAGES * (int)gridDim.x; nt < src.ntiles;
          ++i, nt += gridDim.x) {
         const int s = i % STAGES;
         const int mat = mat_of(src, nt);
@@ -675,7 +680,7 @@ __device__ __forceinline__ void epilogue_warp(const Src &src, const Smem<SIGMA, 
     constexpr int TILE = Layout<SIGMA, VK>::TILE;
     // this warp takes the tiles of parity `par` (the CTA's tiles i = par,
     // par + 2, ...): the carry buffers are double-buffered by that parity
-    for (int i = par, tile = blockIdx.x + par * (int)gridDim.x; tile < src.ntiles;
+    for (int i = par, tile = first_tile(src) + blockIdx.x + par * (int)gridDim.x; tile < src.ntiles;
          i += 2, tile += 2 * (int)gridDim.x) {
         const int p = i & 1;
         const bool ok = ptx::mbar_wait_bounded(sm.cfull(p), (uint32_t)((i / 2) & 1),
@@ -943,16 +948,17 @@ __global__ void tile_partition_quad_kernel(int m, int ntiles, long long tile,
         own_tiles((int)r, rowptr[r], rowptr[r + 1], ntiles, t32, part);
 }
 
-// Adds the carries of the tiles a row spans to the row, in tile order.  (Plain
+// Adds the carries of the tiles a row spans to the row, in tile order, for the
+// rows that end in tiles [k0, ntiles), k0 >= 1.  (Plain
 // pointers: what the kernel before wrote is read after griddep_wait, and a
 // load marked as constant could be moved ahead of it.)
-__global__ void tile_fixup_kernel(int ntiles, long long tile, double alpha, const int *rowptr,
+__global__ void tile_fixup_kernel(int k0, int ntiles, long long tile, double alpha, const int *rowptr,
                                   const int *part, const double *carry, double *y,
                                   const int *status)
 {
     ptx::griddep_launch_dependents();   // the next product may start its set-up
     ptx::griddep_wait();   // launched behind the tile kernel: its carries are complete
-    const int k = blockIdx.x * blockDim.x + threadIdx.x + 1;
+    const int k = blockIdx.x * blockDim.x + threadIdx.x + k0;
     if (k >= ntiles) return;
     if (*status != 0) return;
     const int r = part[k];
@@ -1072,7 +1078,7 @@ int launch_shape(const Src &a, cudaStream_t stream)
     size_t smem = 0;
     const int rc = configure_shape<SIGMA, VK, AB, Src, SKIP>(&bps, &smem);
     if (rc != SBLAS_OK) return rc;
-    const int grid = min(a.ntiles, bps * device_num_sms());
+    const int grid = min(a.ntiles - first_tile(a), bps * device_num_sms());
     SBLAS_CUDA_TRY(launch_pdl(kfn, dim3(grid), dim3(CTA_THREADS), smem, stream, a));
     SBLAS_CUDA_TRY(cudaGetLastError());
     return SBLAS_OK;
@@ -1199,11 +1205,9 @@ int launch_tile_analyse(int m, long long nnz, const int *rowptr, int sigma, void
 // Status word of a tile workspace (after the partition and the carries).
 static int *status_in(void *work) { return static_cast<int *>(work); }
 
-int tile_workspace_status(void *work, int *out)
+int tile_workspace_status(void *work, int *out, cudaStream_t stream)
 {
-    *out = 0;
-    if (work == nullptr) return SBLAS_OK;
-    SBLAS_CUDA_TRY(cudaMemcpy(out, status_in(work), sizeof(int), cudaMemcpyDeviceToHost));
+    SBLAS_CUDA_TRY(cudaMemcpyAsync(out, status_in(work), sizeof(int), cudaMemcpyDeviceToHost, stream));
     return SBLAS_OK;
 }
 
@@ -1336,41 +1340,30 @@ void set_wait_limit_ns(unsigned long long ns)
 
 void set_test_stall(int on) { g_stall.store(on ? 1 : 0, std::memory_order_relaxed); }
 
-int launch_tile_spmv(int m, int n, long long nnz, double alpha, const void *val, int val_kind,
-                     const int *rowptr, const int *col, const double *x, double beta, double *y,
-                     int sigma, void *work, cudaStream_t stream, bool analysed, bool reset_status,
-                     bool skip_zero_x, bool auto_shape)
+int tile_count(long long nnz, int sigma)
 {
-    if (m <= 0) return SBLAS_OK;
-    if (nnz <= 0) return launch_scale_y(m, beta, y, stream);
-    if (auto_shape && small_spmv_fits(m, n, nnz, analysed))
-        return launch_small_spmv(m, alpha, val, val_kind, rowptr, col, x, beta, y,
-                                 reset_status ? status_in(work) : nullptr, stream, skip_zero_x);
-    if (tile_shape_index(sigma) < 0) {
-        set_error(SBLAS_ERR_UNSUPPORTED, "sigma %d is not a compiled tile shape", sigma);
-        return SBLAS_ERR_UNSUPPORTED;
-    }
     const long long tile = (long long)TC * sigma;
-    const long long ntiles_ll = (nnz + tile - 1) / tile;
-    if (ntiles_ll > INT_MAX - 2) {
-        set_error(SBLAS_ERR_ARG, "nnz %lld too large", nnz);
-        return SBLAS_ERR_ARG;
-    }
-    const int ntiles = (int)ntiles_ll;
+    return (int)((nnz + tile - 1) / tile);
+}
+
+int launch_tile_range(int m, int n, long long nnz, double alpha, const void *val, int val_kind,
+                      const int *rowptr, const int *col, const double *x, double beta, double *y,
+                      int sigma, void *work, cudaStream_t stream, int t0, int t1,
+                      bool reset_status, bool skip_zero_x)
+{
+    const long long tile = (long long)TC * sigma;
+    const int ntiles = tile_count(nnz, sigma);
     unsigned char *w = static_cast<unsigned char *>(work);
     int *part = reinterpret_cast<int *>(w + kStatusBytes);
     double *carry = reinterpret_cast<double *>(w + kStatusBytes +
                                                align256(sizeof(int) * (size_t)(ntiles + 1)));
     int *status = status_in(work);
-    if (!analysed) {
-        const int rc = launch_tile_analyse(m, nnz, rowptr, sigma, work, stream);
-        if (rc != SBLAS_OK) return rc;
-    }
     TileArgs a;
     a.m = m;
     a.n = n;
     a.nnz = nnz;
-    a.ntiles = ntiles;
+    a.tile0 = t0;
+    a.ntiles = t1;
     a.alpha = alpha;
     a.beta = beta;
     a.val = val;
@@ -1395,23 +1388,53 @@ int launch_tile_spmv(int m, int n, long long nnz, double alpha, const void *val,
         }
         rc = val_kind == VAL_F64 ? launch_ab<11, VAL_F64, true>(a, stream)
                                  : launch_ab<11, VAL_PATTERN, true>(a, stream);
-    } else switch (sigma) {
-    case 11: rc = launch_vk<11>(val_kind, a, stream); break;
-    case 15: rc = launch_vk<15>(val_kind, a, stream); break;
-    case 19: rc = launch_vk<19>(val_kind, a, stream); break;
-    case 23: rc = launch_vk<23>(val_kind, a, stream); break;
-    case 27: rc = launch_vk<27>(val_kind, a, stream); break;
-    default: rc = SBLAS_ERR_UNSUPPORTED; break;
+    } else {
+        switch (sigma) {
+        case 11: rc = launch_vk<11>(val_kind, a, stream); break;
+        case 15: rc = launch_vk<15>(val_kind, a, stream); break;
+        case 19: rc = launch_vk<19>(val_kind, a, stream); break;
+        case 23: rc = launch_vk<23>(val_kind, a, stream); break;
+        case 27: rc = launch_vk<27>(val_kind, a, stream); break;
+        default: rc = SBLAS_ERR_UNSUPPORTED; break;
+        }
     }
     if (rc != SBLAS_OK) return rc;
-    if (ntiles > 1) {
+    const int k0 = t0 > 1 ? t0 : 1;
+    if (t1 > k0) {
         const int threads = 256;
-        const int blocks = (ntiles - 1 + threads - 1) / threads;
-        SBLAS_CUDA_TRY(launch_pdl(tile_fixup_kernel, dim3(blocks), dim3(threads), 0, stream,
-                                  ntiles, tile, alpha, rowptr, part, carry, y, status));
-        SBLAS_CUDA_TRY(cudaGetLastError());
+        const int blocks = (t1 - k0 + threads - 1) / threads;
+        SBLAS_CUDA_TRY(launch_pdl(tile_fixup_kernel, dim3(blocks), dim3(threads), 0, stream, k0,
+                                  t1, tile, alpha, rowptr, part, carry, y, status));
     }
     return SBLAS_OK;
+}
+
+int launch_tile_spmv(int m, int n, long long nnz, double alpha, const void *val, int val_kind,
+                     const int *rowptr, const int *col, const double *x, double beta, double *y,
+                     int sigma, void *work, cudaStream_t stream, bool analysed, bool reset_status,
+                     bool skip_zero_x, bool auto_shape)
+{
+    if (m <= 0) return SBLAS_OK;
+    if (nnz <= 0) return launch_scale_y(m, beta, y, stream);
+    if (auto_shape && small_spmv_fits(m, n, nnz, analysed))
+        return launch_small_spmv(m, alpha, val, val_kind, rowptr, col, x, beta, y,
+                                 reset_status ? status_in(work) : nullptr, stream, skip_zero_x);
+    if (tile_shape_index(sigma) < 0) {
+        set_error(SBLAS_ERR_UNSUPPORTED, "sigma %d is not a compiled tile shape", sigma);
+        return SBLAS_ERR_UNSUPPORTED;
+    }
+    const long long tile = (long long)TC * sigma;
+    const long long ntiles_ll = (nnz + tile - 1) / tile;
+    if (ntiles_ll > INT_MAX - 2) {
+        set_error(SBLAS_ERR_ARG, "nnz %lld too large", nnz);
+        return SBLAS_ERR_ARG;
+    }
+    if (!analysed) {
+        const int rc = launch_tile_analyse(m, nnz, rowptr, sigma, work, stream);
+        if (rc != SBLAS_OK) return rc;
+    }
+    return launch_tile_range(m, n, nnz, alpha, val, val_kind, rowptr, col, x, beta, y, sigma, work,
+                             stream, 0, (int)ntiles_ll, reset_status, skip_zero_x);
 }
 
 }  // namespace sblas
