@@ -131,7 +131,19 @@ bool check_kernel(const char *name, int kernel)
     return true;
 }
 
-constexpr long long kPipeMinNnz = 1LL << 22;   // smaller matrices: copy, then compute
+// Chunks of a host-array call, 0: copy everything, then compute.  From pinned
+// memory four chunks hide all but a quarter of the kernel.  From pageable
+// memory a copy costs ~13 us beside its bytes and blocks the host, about what
+// the kernel of a chunk saves: one chunk (the partition runs behind the copy of
+// x and of the matrix) up to 16M nonzeros, two above.  Measured, us per call
+// from pageable memory with 0 / 1 / 2 / 4 chunks: 0.85M nonzeros 166 / 157 / 183 /
+// 229, 3.4M 355 / 346 / 366 / 408, 7.0M - / 643 / 645 / 693, 17.5M - / 1436 /
+// 1431 / 1479.
+int host_chunks(long long nnz, bool pinned)
+{
+    if (pinned) return nnz >= (1LL << 22) ? kPipeChunks : 0;
+    return nnz >= (1LL << 24) ? 2 : nnz >= (1LL << 19) ? 1 : 0;
+}
 
 // After the call's stream has completed: false (with SBLAS_ERR_TIMEOUT set)
 // if a tile launch of the call gave up one of its bounded waits (the status
@@ -159,8 +171,7 @@ bool is_pinned(const void *p)
     return a.type == cudaMemoryTypeHost;
 }
 
-// Large CSR calls with host arrays: the matrix travels in kPipeChunks chunks of
-// whole tiles, and the tiles of a chunk run as soon as its values and columns
+// Large CSR calls with host arrays: the matrix travels in K chunks of whole tiles, and the tiles of a chunk run as soon as its values and columns
 // have arrived (copies on the context's copy stream, kernels on its compute
 // stream), so the kernels hide behind the host-to-device copies, which the host
 // link bounds.  A copy from pageable memory blocks the host until it is done:
@@ -169,11 +180,10 @@ bool is_pinned(const void *p)
 // arrived, 820 us per call with 7.7M nonzeros).  One partition serves all
 // chunks; they share the row pointer as it is.  y goes back chunk by chunk from
 // pinned memory, in one copy at the end to pageable memory.
-spmv_ret run_host_pipelined(const Call &c, DeviceContext *ctx)
+spmv_ret run_host_pipelined(const Call &c, DeviceContext *ctx, int K)
 {
     const int m = c.m, n = c.n;
     const long long nnz = c.nnz;
-    const int K = kPipeChunks;
     const bool need_y_in = (c.beta != 0.0) || c.additive;
     cudaStream_t cs = ctx->copy_stream, ks = ctx->stream;
     const int sigma = (c.kernel == 3) ? csr5_sigma_for(m, nnz) : default_sigma_for(m, nnz);
@@ -256,9 +266,10 @@ spmv_ret run_host(Call c)
     }
     spmv_ret ret = zero_ret();
     if (c.m == 0) return ret;
-    if (c.fmt == Fmt::CSR && c.kernel != 1 && c.nnz >= kPipeMinNnz && c.n > 0 && c.row_lo == 0 &&
-        c.row_hi == c.m)
-        return run_host_pipelined(c, ctx);
+    if (c.fmt == Fmt::CSR && c.kernel != 1 && c.n > 0 && c.row_lo == 0 && c.row_hi == c.m) {
+        const int K = host_chunks(c.nnz, c.nnz > 0 && is_pinned(c.val));
+        if (K > 0) return run_host_pipelined(c, ctx, K);
+    }
     cudaStream_t st = ctx->stream;
     const int m = c.m, n = c.n;
     const long long nnz = c.nnz;

@@ -181,3 +181,30 @@ def test_small_matrices(sblas_lib, cuda, lengths):
                                      beta, sigma=15)
             for what, y in got.items():
                 assert rel_l2(y.cpu().numpy(), ref) <= RTOL_L2, (form, what, alpha, beta)
+
+
+@pytest.mark.parametrize("pinned", [False, True])
+@pytest.mark.parametrize("nnz", [(1 << 19) - 1, 1 << 19, (1 << 22) - 1, 1 << 22, (1 << 24) + 5])
+def test_host_call_chunks(sblas_lib, cuda, pinned, nnz):
+    """Host arrays on both sides of each chunk count, pageable and pinned, a row
+    over several chunks, empty rows at both ends, beta with y read in."""
+    from hpda_sblas_pnnl_gb300 import api
+    rng = np.random.default_rng(nnz)
+    m, n = nnz // 50, 40_000
+    lengths = rng.multinomial(nnz - nnz // 3, np.ones(m) / m)
+    lengths[:3] = 0
+    lengths[-4:] = 0
+    lengths[m // 3] += nnz - int(lengths.sum())
+    rp = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
+    col = rng.integers(0, n, nnz).astype(np.int32)
+    val, x, y0 = rng.standard_normal(nnz), rng.standard_normal(n), rng.standard_normal(m)
+    y = y0.copy()
+    if pinned:
+        keep = [torch.from_numpy(a).pin_memory() for a in (val, rp, col, x, y)]
+        val, rp, col, x, y = (t.numpy() for t in keep)
+    for alpha, beta in ((1.0, 0.0), (1.5, -0.5)):
+        y[:] = y0
+        api.spMV_mgpu_v1(m, n, nnz, alpha, val, rp, col, x, beta, y)
+        ref = O.csr_spmv(m, n, np.array(rp), np.array(col), np.array(val), np.array(x), y0.copy(),
+                         alpha, beta)
+        assert rel_l2(y, ref) <= RTOL_L2
