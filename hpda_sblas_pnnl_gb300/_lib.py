@@ -136,6 +136,7 @@ SIGNATURES: dict[str, tuple] = {
     "sblas_gather_values": (C.c_int, [C.c_longlong, C.c_int, _vp, _vp, _vp, _vp]),
     "sblas_zero": (C.c_int, [_vp, C.c_size_t, _vp]),
     "sblas_csr_filter_x_workspace_bytes": (C.c_size_t, [C.c_longlong]),
+    "sblas_dspmspv_workspace_bytes": (C.c_size_t, [C.c_int, C.c_int, C.c_longlong]),
     "sblas_dspmspv": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_longlong, C.c_double, _vp, _vp,
                                 _vp, _vp, C.c_double, _vp, _vp, C.c_size_t, _vp]),
     "sblas_csr_filter_x": (C.c_int, [C.c_int, C.c_longlong, _vp, _vp, _vp, _vp, _vp, _vp, _vp,

@@ -404,6 +404,12 @@ int sblas_csr_filter_x(int m, long long nnz, const int *rowptr, const int *col,
                                work_bytes, static_cast<cudaStream_t>(stream));
 }
 
+size_t sblas_dspmspv_workspace_bytes(int m, int n, long long nnz)
+{
+    if (nnz <= 0 || m <= 0 || small_spmv_fits(m, n, nnz, false)) return 0;
+    return tile_workspace_bytes(nnz, default_sigma_for(m, nnz));
+}
+
 int sblas_dspmspv(int kernel, int m, int n, long long nnz, double alpha, const double *val,
                   const int *rowptr, const int *col, const double *x, double beta, double *y,
                   void *work, size_t work_bytes, void *stream)
@@ -434,14 +440,14 @@ int sblas_dspmspv(int kernel, int m, int n, long long nnz, double alpha, const d
         return launch_rowsplit_spmv(m, n, nnz, alpha, val, rowptr, col, x, beta, y, st, true);
     }
     const int sigma = default_sigma_for(m, nnz);
-    const size_t need = tile_workspace_bytes(nnz, sigma);
-    if (nnz > 0 && (work == nullptr || work_bytes < need ||
+    const size_t need = sblas_dspmspv_workspace_bytes(m, n, nnz);
+    if (need > 0 && (work == nullptr || work_bytes < need ||
                     (reinterpret_cast<uintptr_t>(work) & 255) != 0)) {
         set_error(SBLAS_ERR_ARG, "workspace needs %zu bytes at 256-byte alignment", need);
         return SBLAS_ERR_ARG;
     }
     return launch_tile_spmv(m, n, nnz, alpha, val, val ? VAL_F64 : VAL_PATTERN, rowptr, col, x,
-                            beta, y, sigma, work, st, false, true, true, true);
+                            beta, y, sigma, work, st, false, need > 0, true, true);
 }
 
 int sblas_zero(void *p, size_t bytes, void *stream)

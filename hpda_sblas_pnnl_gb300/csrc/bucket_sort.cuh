@@ -34,6 +34,7 @@
 // with 4.5M entries: 275 -> 188 us.
 #pragma once
 
+#include <atomic>
 #include <climits>
 
 #include "launch.cuh"
@@ -695,14 +696,19 @@ int count_digits(const int *key, long long n, int shift, int nb, const PassTable
     return SBLAS_OK;
 }
 
-// A kernel's dynamic shared memory and the largest carveout: these kernels'
-// loads stream, nothing they read is reused through L1.
+// A kernel's dynamic shared memory and the largest carveout (these kernels'
+// loads stream, nothing they read is reused through L1), set once per device.
 template <class K>
-int allow_smem(K kfn, size_t bytes)
+int allow_smem(K kfn, size_t bytes, std::atomic<unsigned long long> &done)
 {
+    int dev = 0;
+    SBLAS_CUDA_TRY(cudaGetDevice(&dev));
+    const unsigned long long bit = dev >= 0 && dev < 64 ? 1ull << dev : 0;
+    if (bit != 0 && (done.load(std::memory_order_acquire) & bit) != 0) return SBLAS_OK;
     SBLAS_CUDA_TRY(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
     SBLAS_CUDA_TRY(cudaFuncSetAttribute(kfn, cudaFuncAttributePreferredSharedMemoryCarveout,
                                         (int)cudaSharedmemCarveoutMaxShared));
+    done.fetch_or(bit, std::memory_order_release);
     return SBLAS_OK;
 }
 
@@ -720,7 +726,8 @@ int scatter_pass_iter(const Arrays &op, long long n, int shift, int nb, void *wo
     int rc = count_digits<ITER>(op.key_in, n, shift, nb, t, stream);
     if (rc != SBLAS_OK) return rc;
     auto kfn = bucket_scatter_kernel<SEG, IDX, POS, ITER>;
-    rc = allow_smem(kfn, scatter_smem_bytes<ITER>(MAXB));
+    static std::atomic<unsigned long long> configured{0};
+    rc = allow_smem(kfn, scatter_smem_bytes<ITER>(MAXB), configured);
     if (rc != SBLAS_OK) return rc;
     SBLAS_CUDA_TRY(launch_pdl(kfn, dim3((unsigned)t.tiles), dim3(THREADS),
                               scatter_smem_bytes<ITER>(table_width(nb)), stream, op, n, shift,
