@@ -72,9 +72,10 @@ bool s_compiled(int s) { return s == 4 || s == 8 || s == 16 || s == 32; }
 //            nnz      s = 1         2         4         8        16        32
 //   k = 1   8e3                       7.5/6.3   9.1/6.3  12.4/8.3
 //           2.0e7                     162/164   139/112   166/144   161/132
-//   k = 2   1.6e6                      31/28     26/19     29/22     27/24
-//           3.1e6 (6 per row)          64/43     56/32     60/34
-//           2.0e7                     231/275   174/161   168/165   248/262
+//   k = 2   6.2e5                      22/18     19/15     19/15
+//           3.1e6 (6 per row)          61/37     54/29     54/29
+//           1.6e7 (80 per row)        179       133       126
+//           2.0e7                     234/277   165/152   151/147
 //   k = 4   1.6e5                    14.8/10.3 14.0/10.3 15.7/12.8
 //           6.2e5                    23.6/22.6 21.0/18.1 18.1/16.1 22.6/18.5
 //           2.0e7                     380/487   292/297   249/230   335/321
@@ -100,7 +101,7 @@ int pick_s(int k, long long nnz, bool permuted_f64)
         return nnz < (1 << 14) ? 1 : nnz < 200000 ? 2 : nnz < 1000000 ? 4
                : nnz < 6000000 || permuted_f64 ? 8 : 16;
     if (nnz < (1 << 14)) return 4;
-    return k == 4 && nnz >= 400000 ? 16 : 8;
+    return (k == 4 && nnz >= 400000) || (k == 2 && nnz >= 2000000) ? 16 : 8;
 }
 
 bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }

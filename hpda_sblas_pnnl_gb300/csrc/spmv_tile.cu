@@ -956,7 +956,6 @@ __global__ void tile_fixup_kernel(int k0, int ntiles, long long tile, double alp
                                   const int *part, const double *carry, double *y,
                                   const int *status)
 {
-    ptx::griddep_launch_dependents();   // the next product may start its set-up
     ptx::griddep_wait();   // launched behind the tile kernel: its carries are complete
     const int k = blockIdx.x * blockDim.x + threadIdx.x + k0;
     if (k >= ntiles) return;
@@ -983,7 +982,6 @@ __global__ void scale_y_kernel(int m, double beta, double *__restrict__ y)
 // own tiles and partition.
 __global__ void multi_fixup_kernel(const MultiArgs a, long long tile)
 {
-    ptx::griddep_launch_dependents();
     ptx::griddep_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.ntiles) return;
