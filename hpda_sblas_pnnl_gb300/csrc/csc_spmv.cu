@@ -16,10 +16,9 @@
 //   sorted     the one-shot product, whose inspector runs on every call, lets
 //              the sort carry the values instead of the positions (a gather by
 //              position afterwards cost 24 us more on 4.5M entries);
-//   direct     out[p] = val[perm[p]], for an analysed pattern of one bucket
-//              (its values stay in L2);
-//   staged     for an analysed pattern reused many times (sblas_csc_analyse):
-//              the row-order positions are cut into buckets of 2^bits
+//   direct     out[p] = val[perm[p]], for an analysed pattern
+//              (sblas_csc_analyse) of up to 2^25 entries;
+//   staged     for a larger one: the row-order positions are cut into buckets of 2^bits
 //              (8 MB of values).  The inspector adds two index arrays:
 //              dst[q], the slot of CSC entry q in a staging array that holds
 //              every bucket's values contiguously (in CSC order inside the
@@ -45,6 +44,13 @@ size_t al256(size_t v) { return (v + 255) & ~size_t(255); }
 
 constexpr int kCscSigma = 11;     // tile shape of the executor (the library default)
 constexpr int kStageBits = 20;    // staging bucket: 2^20 row positions (8 MB of values)
+// Up to here the values are gathered directly: even past the L2 (2^24 values)
+// one gather beats the two staged moves until nearly every read of a pattern
+// without locality goes to DRAM.  Product with new values, us, staged / direct:
+// power-law 4.0M entries 68 / 52, 12M 164 / 127, 20M 258 / 224, 24M 305 / 285,
+// 30M 376 / 382, 40M 499 / 549, 60M 750 / 913; banded 6.1M 82 / 60, 20M 214 / 155,
+// 32M 330 / 238, 39M 406 / 294.
+constexpr long long kStageMin = 1LL << 25;
 constexpr int kStageBuckets = 256;   // at most (the bucket pass's digit values)
 constexpr int kStageIter = 8;     // entries per thread of the staging pass's tiles
 
@@ -57,7 +63,7 @@ struct StagePlan {
 StagePlan stage_plan(long long nnz)
 {
     StagePlan s{kStageBits, 1, 1};
-    if (nnz <= 1) return s;
+    if (nnz <= kStageMin) return s;
     while (((nnz - 1) >> s.bits) >= kStageBuckets) ++s.bits;
     s.used = (int)(((nnz - 1) >> s.bits) + 1);
     while (s.nb < s.used) s.nb <<= 1;

@@ -208,3 +208,59 @@ def test_host_call_chunks(sblas_lib, cuda, pinned, nnz):
         ref = O.csr_spmv(m, n, np.array(rp), np.array(col), np.array(val), np.array(x), y0.copy(),
                          alpha, beta)
         assert rel_l2(y, ref) <= RTOL_L2
+
+
+@pytest.mark.parametrize("nnz", [1, 3, 4, 5, 127, 4095, 4096, 4097, 8191, 131_073, 300_001])
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("m", [1, 700, 200_000])
+def test_coo_row_pointer_and_partition(sblas_lib, cuda, nnz, offset, m):
+    """Sorted triplets at the edges of the row-pointer kernel's CTAs and of the
+    tiles, aligned and not, rows missing at both ends and between, one row over
+    many tiles: the row pointer equal, products within the bar, every shape."""
+    from hpda_sblas_pnnl_gb300 import ops
+    rng = np.random.default_rng(nnz + m)
+    n = 500
+    rows = np.sort(rng.integers(m // 3, max(m - m // 5, m // 3 + 1), nnz)).astype(np.int32)
+    rows[nnz // 4: nnz // 2] = rows[nnz // 4]
+    rows = np.sort(rows)
+    col = rng.integers(0, n, nnz).astype(np.int32)
+    val, x = rng.standard_normal(nnz), rng.standard_normal(n)
+    y0 = rng.standard_normal(m)
+    pad = torch.zeros(nnz + offset, dtype=torch.int32, device=cuda)
+    pad[offset:] = torch.from_numpy(rows).to(cuda)
+    tr = pad[offset:]
+    tc, tv, tx = (torch.from_numpy(a).to(cuda) for a in (col, val, x))
+    ref = O.coo_spmv(m, n, rows, col, val, x, y0.copy(), 1.5, -0.5)
+    for sigma in (0, 11, 27):
+        y = torch.from_numpy(y0).to(cuda)
+        work = torch.full((m + 1,), -7, dtype=torch.int32, device=cuda)
+        ops.coomv(tr, tc, tv, tx, y, 1.5, -0.5, rowptr_work=work, sigma=sigma)
+        assert rel_l2(y.cpu().numpy(), ref) <= RTOL_L2
+        want = np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=m))])
+        assert np.array_equal(work.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("nnz", [1 << 20, (1 << 25) - 3, 1 << 25, (1 << 25) + 5])
+def test_csc_values_direct_and_staged(sblas_lib, cuda, nnz):
+    """An analysed CSC pattern on both sides of the size from which its values
+    are staged: new values, bound values, against the one-shot product."""
+    from hpda_sblas_pnnl_gb300 import ops
+    g = torch.Generator(device=cuda)
+    g.manual_seed(nnz)
+    m, n = nnz // 40, nnz // 30
+    rows = torch.randint(0, m, (nnz,), generator=g, device=cuda, dtype=torch.int32)
+    cols = torch.sort(torch.randint(0, n, (nnz,), generator=g, device=cuda)).values
+    colptr = torch.zeros(n + 1, dtype=torch.int64, device=cuda)
+    colptr[1:] = torch.cumsum(torch.bincount(cols, minlength=n), 0)
+    colptr = colptr.int()
+    x = torch.randn(n, generator=g, dtype=torch.float64, device=cuda)
+    plan = ops.CscPlan(m, colptr, rows)
+    for _ in range(2):
+        val = torch.randn(nnz, generator=g, dtype=torch.float64, device=cuda)
+        ref = torch.zeros(m, dtype=torch.float64, device=cuda).index_add_(0, rows.long(), val * x[cols])
+        once = ops.cscmv(colptr, rows, val, x, torch.empty_like(ref))
+        assert float((once - ref).norm() / ref.norm()) <= RTOL_L2
+        y = plan(val, x, torch.empty_like(ref))
+        assert torch.equal(y, once)
+        plan.bind(val)
+        assert torch.equal(plan(None, x, torch.empty_like(ref)), once)
