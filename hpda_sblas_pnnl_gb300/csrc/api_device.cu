@@ -152,12 +152,15 @@ int sblas_tile_sigma_at(int i)
 int sblas_default_sigma(int m, long long nnz) { return default_sigma_for(m, nnz); }
 int sblas_csr5_sigma(int m, long long nnz) { return csr5_sigma_for(m, nnz); }
 
-int sblas_dcsrmv(int kernel, int m, int n, long long nnz, double alpha, const void *val,
+}  // extern "C"
+
+// sblas_dcsrmv; with coo_row, the row pointer is not there yet and is made from
+// those row indices (into coo_rowptr == rowptr) once the arguments are known.
+static int csrmv(int kernel, int m, int n, long long nnz, double alpha, const void *val,
                  int val_kind, const int *rowptr, const int *col, const double *x, double beta,
-                 double *y, int sigma, void *work, size_t work_bytes, void *stream)
+                 double *y, int sigma, void *work, size_t work_bytes, cudaStream_t st,
+                 const int *coo_row, int *coo_rowptr)
 {
-    clear_error();
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (m < 0 || n < 0 || nnz < 0 || nnz > 0x7fffffffLL) {
         set_error(SBLAS_ERR_ARG, "bad sizes m=%d n=%d nnz=%lld", m, n, nnz);
         return SBLAS_ERR_ARG;
@@ -200,8 +203,28 @@ int sblas_dcsrmv(int kernel, int m, int n, long long nnz, double alpha, const vo
         set_error(SBLAS_ERR_ARG, "workspace needs %zu bytes at 256-byte alignment", need);
         return SBLAS_ERR_ARG;
     }
+    bool analysed = false;
+    if (coo_row != nullptr) {   // a row index per nonzero gives the partition too
+        analysed = nnz > 0 && tile_shape_index(sigma) >= 0 && coo_partition_fits(coo_row) &&
+                   !(auto_shape && small_spmv_fits(m, n, nnz, false));
+        const int rc = launch_coo_rows_to_rowptr(m, nnz, coo_row, coo_rowptr, st, sigma,
+                                                 analysed ? work : nullptr);
+        if (rc != SBLAS_OK) return rc;
+    }
+    const bool small = auto_shape && small_spmv_fits(m, n, nnz, false);
     return launch_tile_spmv(m, n, nnz, alpha, val, val_kind, rowptr, col, x, beta, y, sigma,
-                            work, st, false, true, false, auto_shape);
+                            work, st, analysed, true, false, small);
+}
+
+extern "C" {
+
+int sblas_dcsrmv(int kernel, int m, int n, long long nnz, double alpha, const void *val,
+                 int val_kind, const int *rowptr, const int *col, const double *x, double beta,
+                 double *y, int sigma, void *work, size_t work_bytes, void *stream)
+{
+    clear_error();
+    return csrmv(kernel, m, n, nnz, alpha, val, val_kind, rowptr, col, x, beta, y, sigma, work,
+                 work_bytes, static_cast<cudaStream_t>(stream), nullptr, nullptr);
 }
 
 int sblas_csr_analyse(int kernel, int m, long long nnz, const int *rowptr, int sigma, void *work,
@@ -264,10 +287,17 @@ int sblas_dcoomv(int m, int n, long long nnz, double alpha, const double *val,
         return SBLAS_ERR_ARG;
     }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    int rc = launch_coo_rows_to_rowptr(m, nnz, coo_row, rowptr_work, st);
-    if (rc != SBLAS_OK) return rc;
-    return sblas_dcsrmv(SBLAS_KERNEL_MERGEPATH, m, n, nnz, alpha, val, SBLAS_VAL_F64,
-                        rowptr_work, coo_col, x, beta, y, sigma, work, work_bytes, stream);
+    if (nnz > 0 && coo_row == nullptr) {
+        set_error(SBLAS_ERR_ARG, "null device pointer");
+        return SBLAS_ERR_ARG;
+    }
+    if (m == 0 || nnz == 0) {   // the row pointer of an empty matrix
+        const int rc = launch_coo_rows_to_rowptr(m, nnz, coo_row, rowptr_work, st);
+        if (rc != SBLAS_OK) return rc;
+        coo_row = nullptr;
+    }
+    return csrmv(SBLAS_KERNEL_MERGEPATH, m, n, nnz, alpha, val, SBLAS_VAL_F64, rowptr_work, coo_col,
+                 x, beta, y, sigma, work, work_bytes, st, coo_row, rowptr_work);
 }
 
 size_t sblas_csc_to_csr_workspace_bytes(int m, int n, long long nnz)

@@ -1344,6 +1344,11 @@ int tile_count(long long nnz, int sigma)
     return (int)((nnz + tile - 1) / tile);
 }
 
+int *tile_workspace_part(void *work)
+{
+    return reinterpret_cast<int *>(static_cast<unsigned char *>(work) + kStatusBytes);
+}
+
 int launch_tile_range(int m, int n, long long nnz, double alpha, const void *val, int val_kind,
                       const int *rowptr, const int *col, const double *x, double beta, double *y,
                       int sigma, void *work, cudaStream_t stream, int t0, int t1,
