@@ -281,7 +281,6 @@ __global__ void __launch_bounds__(CTA) batch_spmm_kernel(const Args a)
     double *hbuf = reinterpret_cast<double *>(ws + WS::HBUF) + lane * KP;
     const uint64_t pol_x = ptx::policy_evict_last();
     const unsigned FULL = 0xffffffffu;
-    ptx::griddep_launch_dependents();   // the fix-up may start (it waits for this grid's end)
 
     for (int u = blockIdx.x * NW + warp; u < a.nunits; u += gridDim.x * NW) {
         const int b = __ldg(a.unit_mat + u);
@@ -655,7 +654,6 @@ __global__ void __launch_bounds__(CTA, 8) batch_spmm_vec_kernel(const Args a)
     int *mtrow = mhrow + G;
     int *mmid = mtrow + G;
     const uint64_t pol_x = ptx::policy_evict_last();
-    ptx::griddep_launch_dependents();   // the fix-up may start (it waits for this grid's end)
 
     for (int u = blockIdx.x * NW + warp; u < a.nunits; u += gridDim.x * NW) {
         const int b = __ldg(a.unit_mat + u);

@@ -819,7 +819,6 @@ __global__ void __launch_bounds__(CTA_THREADS, min_ctas<SIGMA, VK>())
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
     const int lane = tid & 31;
-    ptx::griddep_launch_dependents();   // the fix-up's CTAs may wait beside this grid's
     if (tid == 0) {
         for (int s = 0; s < STAGES; ++s) {
             ptx::mbar_init(sm.full(s), 1);
@@ -834,8 +833,13 @@ __global__ void __launch_bounds__(CTA_THREADS, min_ctas<SIGMA, VK>())
     for (int i = tid; i < 2 * L::RCAP; i += CTA_THREADS) sm.rval(0)[i] = 0.0;
     __syncthreads();
     // launched right behind the tile partition (or the fix-up of the product
-    // before): the set-up above overlapped its end; nothing in global memory is
-    // touched before it has finished
+    // before) with programmatic stream serialisation, which saves the launch
+    // latency between them.  No kernel of this chain lets its successor start
+    // early (griddep_launch_dependents): the waiting CTAs then take registers
+    // and thread slots beside the ones that run, and tile CTAs are placed
+    // around them unevenly.  With early starts / without: analysed product,
+    // banded 6.4M nonzeros FP32 26.9 / 24.3 us, 17M power-law 87.0 / 85.0;
+    // per call 32.1 / 29.0, 94.9 / 91.7; batch k = 1 141 / 91 us.
     ptx::griddep_wait();
     // The status word is cleared here, not by a memset of its own (a launch
     // and ~1 us per product): a wait of this launch can give up and report at
@@ -898,7 +902,6 @@ __global__ void tile_partition_kernel(int m, long long nnz, int ntiles, long lon
                                       const int *rowptr, int *part)
 {
     (void)nnz;
-    ptx::griddep_launch_dependents();   // the tile kernel may start its set-up
     const int stride = gridDim.x * blockDim.x;
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g == 0) {
@@ -917,7 +920,6 @@ __global__ void tile_partition_quad_kernel(int m, int ntiles, long long tile,
                                            const int *rowptr,
                                            int *part)
 {
-    ptx::griddep_launch_dependents();   // the tile kernel may start its set-up
     const long long stride = (long long)gridDim.x * blockDim.x;
     const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (g == 0) {
@@ -1185,9 +1187,8 @@ int launch_tile_analyse(int m, long long nnz, const int *rowptr, int sigma, void
     const int ntiles = (int)ntiles_ll;
     int *part = reinterpret_cast<int *>(static_cast<unsigned char *>(work) + kStatusBytes);
     const int threads = 256;
-    // An ordinary launch: as a programmatic dependent of the product before, its
-    // CTAs sat beside that product's and the next tile kernel's CTAs were placed
-    // around them, unevenly over the SMs (power-law step 388 -> 501 us).
+    // An ordinary launch (as a programmatic dependent of the product before:
+    // power-law step 388 -> 501 us, see tile_spmv_kernel).
     if ((reinterpret_cast<uintptr_t>(rowptr) & 15) == 0) {
         const int quads = m / 4 + 1;
         const int blocks = min((quads + threads - 1) / threads, 8 * device_num_sms());
