@@ -937,6 +937,20 @@ __global__ void __launch_bounds__(FIX_THREADS) batch_fixup_kernel(const Args a)
     }
 }
 
+// Independent partial sums of a value's K products.  Each one more costs the
+// FP64 pipe, which bounds this kernel, an add per nonzero; each one fewer makes
+// the chain of dependent multiply-adds (~65 cycles each) longer, which the other
+// warps cover.  As few as leave the sum's rounding error where it was with four.
+// With 4 / 2 / 1 sums over 2.0e7 nonzeros, and the relative error for normal and
+// for uniform factors in units of 1e-17:
+//   K = 4   218 / 215 / 166 us   8.5 / 7.6 / 7.5    7.1 / 6.7 / 6.6
+//   K = 8   456 / 369 / 307 us   9.2 / 9.0 / 10.0   7.27 / 7.30 / 8.6
+//   K = 16  730 / 746 / 655 us   10.4 / 11.2 / 13.7 (normal)
+// (Adding the first products to zero instead of starting the sums with them
+// took 292 us for K = 4.)
+template <int K>
+constexpr int sddmm_parts() { return K <= 4 ? 1 : K == 8 ? 2 : 4; }
+
 // ---- sampled dense-dense product over the pattern (values' adjoint) -------
 // dval[p] = sum over c of G[row(p), c] * X[col(p), c] for every stored entry
 // of a single-matrix plan; one warp per unit, lane l takes nonzeros
@@ -965,6 +979,7 @@ __global__ void __launch_bounds__(CTA) batch_sddmm_kernel(const Args a)
         }
         int r = lo;
         int next = __ldg(rowptr + r + 1);
+        constexpr int NP = sddmm_parts<K>();
         for (int i = lane; i < cntu; i += 32, p += 32) {
             while (next <= p) {
                 ++r;
@@ -973,15 +988,11 @@ __global__ void __launch_bounds__(CTA) batch_sddmm_kernel(const Args a)
             double gr[K], xr[K];
             gather_row<K>(a.g, out_row(M, r), a.ldg, gr, pol);
             gather_row<K>(a.x, __ldcs(col + p), a.ldx, xr, pol);
-            // four independent partial sums, joined at the end: the dependent
-            // DFMA latency is long on this GPU (two partial sums, one join
-            // less, measured slower: 0.70 -> 0.76 ms on the autograd matrix)
-            constexpr int NP = K >= 4 ? 4 : K;
             double part[NP];
 #pragma unroll
-            for (int q = 0; q < NP; ++q) part[q] = 0.0;
+            for (int h = 0; h < NP; ++h) part[h] = gr[h] * xr[h];
 #pragma unroll
-            for (int c = 0; c < K; ++c) part[c % NP] = fma(gr[c], xr[c], part[c % NP]);
+            for (int c = NP; c < K; ++c) part[c % NP] = fma(gr[c], xr[c], part[c % NP]);
             double d;
             if constexpr (NP == 4) d = (part[0] + part[1]) + (part[2] + part[3]);
             else if constexpr (NP == 2) d = part[0] + part[1];
