@@ -80,6 +80,32 @@ def test_plan_picks_a_shape_for_every_size(sblas_lib, cuda, k, nnz):
                                                    x.cpu().numpy())) <= RTOL_L2
 
 
+@pytest.mark.parametrize("sigma", [11, 27])
+def test_tile_fixup_row_spans(sblas_lib, cuda, sigma):
+    """Rows over 2, 3, 9, 10, 11 and 40 tiles, rows that start or end at a tile
+    boundary, one matrix and several in a launch."""
+    from hpda_sblas_pnnl_gb300 import ops
+    tile = 128 * sigma
+    lengths = [3, tile - 3, tile, 1, 0, 2 * tile - 1, 5, 9 * tile, 10 * tile - 5, 11 * tile + 2, 0,
+               0, 40 * tile, 7, 3 * tile + 1, tile, tile, 2, 2 * tile]
+    n = 4000
+    (rp, col, val), dev = csr_of_lengths(lengths, n, sigma, cuda)
+    m = len(lengths)
+    rng = np.random.default_rng(sigma)
+    x, y0 = rng.standard_normal(n), rng.standard_normal(m)
+    ref = O.csr_spmv(m, n, rp, col, val, x, y0.copy(), 1.5, -0.5)
+    tx = torch.from_numpy(x).to(cuda)
+    y = torch.from_numpy(y0).to(cuda)
+    ops.CsrPlan(*dev, n=n, sigma=sigma)(tx, y, 1.5, -0.5)
+    assert rel_l2(y.cpu().numpy(), ref) <= RTOL_L2
+    if sigma != 11:
+        return                    # several matrices in a launch: one compiled shape
+    ys = [torch.from_numpy(y0).to(cuda) for _ in range(3)]
+    ops.BatchPlan([dev] * 3, [tx] * 3, ys, 1, alpha=1.5, beta=-0.5)()
+    for y in ys:
+        assert rel_l2(y.cpu().numpy(), ref) <= RTOL_L2
+
+
 @pytest.mark.parametrize("kernel", [1, 2, 3])
 @pytest.mark.parametrize("lengths", [[1], [0, 0, 1408, 0], [1407, 1, 1], [1409], [0] * 700 + [3],
                                      [2, 0, 9000, 1, 0, 0, 40, 1500, 7] * 3], ids=str)
