@@ -30,8 +30,8 @@
 // digits.  Equal digits by ballots rather than __match_any_sync, which takes a
 // warp's distinct values one after another: 312 -> 289 us in a copy of the
 // pass; CTAs of 512 threads (twice the warp-private tables): 326 us.
-// CSC to CSR, 20M entries, 1M rows: 890 -> 619 us; one product of a CSC matrix
-// with 4.5M entries: 275 -> 188 us.
+// CSC to CSR, 20M entries, 1M rows: 890 -> 608 us; one product of a CSC matrix
+// with 4.5M entries: 275 -> 171 us.
 #pragma once
 
 #include <atomic>
@@ -46,7 +46,10 @@ namespace bsort {
 // The kernels here are launched behind one another with programmatic stream
 // serialisation and read what the kernel before wrote.  Those reads are plain
 // loads (no __restrict__, no __ldg): a load marked as reading constant memory
-// could be moved ahead of the wait for that kernel.
+// could be moved ahead of the wait for that kernel.  (None of them lets its
+// successor start before its last CTA exits: with early starts the waiting CTAs
+// take slots and shared memory from the running ones, 20M entries 608 -> 617
+// us, 4.5M 144 -> 148, small sorts the same.)
 // internal linkage: every translation unit that includes this header gets its
 // own copy of the kernels (no relocatable device code)
 namespace {
@@ -54,7 +57,7 @@ namespace {
 constexpr int NW = 8;                   // warps per CTA
 constexpr int THREADS = NW * 32;
 constexpr int MAXB = 2048;              // digit values per pass (11-bit digits)
-constexpr int CHUNK_DIGITS = 32;        // digits per CTA of the chunk scan
+constexpr int CHUNK_DIGITS = 8;         // digits per CTA of the chunk scan
 
 // Entries per thread of a pass over n entries: 16 (tiles of 4096, about four
 // entries per run at 1024 digits), or fewer where that would leave the three
@@ -67,10 +70,12 @@ inline long long num_tiles(long long n, int iter)
     return (n + t - 1) / t;
 }
 
-// Tiles per chunk of the digit counts: about a thousand chunks.
+constexpr int MAX_CHUNKS = 1024;        // of the digit counts (bucket_chunks_kernel)
+
+// Tiles per chunk of the digit counts: at most MAX_CHUNKS chunks.
 inline int chunk_tiles(long long ntiles)
 {
-    long long c = (ntiles + 1023) / 1024;
+    long long c = (ntiles + MAX_CHUNKS - 1) / MAX_CHUNKS;
     return (int)(c < 1 ? 1 : c);
 }
 
@@ -170,7 +175,6 @@ __global__ void __launch_bounds__(THREADS) bucket_hist_kernel(const int *key,
 {
     constexpr int T = THREADS * ITER;
     __shared__ int cnt[MAXB];
-    ptx::griddep_launch_dependents();
     const int width = table_width(nb);
     for (int d = threadIdx.x; d < width; d += THREADS) cnt[d] = 0;
     __syncthreads();
@@ -195,46 +199,49 @@ __global__ void __launch_bounds__(THREADS) bucket_hist_kernel(const int *key,
 }
 
 // Per digit: chunk_sum becomes the exclusive prefix over the chunks, total[d]
-// their sum.  A CTA takes 32 digits, a row of 32 threads a span of chunks.
-__global__ void __launch_bounds__(1024) bucket_chunks_kernel(int width, int nchunks,
-                                                             int *chunk_sum,
-                                                             int *total)
+// their sum.  A CTA takes eight digits (32 bytes of a row), eight threads a span
+// of chunks, all of its counts read at once and kept in registers: there is
+// little to do here but wait for memory, so the round trips count.  4.5M
+// entries, two passes: 10 us less than with every span read twice, eight counts
+// at a time, by 1024-thread CTAs of 32 digits; such CTAs with the counts in
+// registers need a whole idle SM each and cost 14 us more.
+__global__ void __launch_bounds__(32 * CHUNK_DIGITS) bucket_chunks_kernel(int width, int nchunks,
+                                                                          int *chunk_sum,
+                                                                          int *total)
 {
-    __shared__ int part[32][33];
-    ptx::griddep_launch_dependents();
+    constexpr int SPAN = MAX_CHUNKS / 32;
+    __shared__ int part[32][CHUNK_DIGITS + 1];
     ptx::griddep_wait();
-    const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
-    const int d = blockIdx.x * CHUNK_DIGITS + lane;
-    const int per = (nchunks + 31) / 32;
-    const int c0 = min(g * per, nchunks), c1 = min(c0 + per, nchunks);
+    const int j = threadIdx.x % CHUNK_DIGITS, g = threadIdx.x / CHUNK_DIGITS;
+    const int d = blockIdx.x * CHUNK_DIGITS + j;
+    const int per = (nchunks + 31) / 32;      // <= SPAN
+    const int c0 = min(g * per, nchunks), c1 = d < width ? min(c0 + per, nchunks) : c0;
+    int x[SPAN];
     int s = 0;
-    if (d < width) {
-#pragma unroll 8
-        for (int c = c0; c < c1; ++c) s += chunk_sum[(long long)c * width + d];
-    }
-    part[g][lane] = s;
+#pragma unroll
+    for (int i = 0; i < SPAN; ++i) x[i] = c0 + i < c1 ? chunk_sum[(long long)(c0 + i) * width + d] : 0;
+#pragma unroll
+    for (int i = 0; i < SPAN; ++i) s += x[i];
+    part[g][j] = s;
     __syncthreads();
-    // warp g scans the 32 spans of digit g of this CTA
-    int v = part[lane][g];
+    // warp w scans the 32 spans of digit w of this CTA
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int v = part[lane][w];
     const int own = v;
 #pragma unroll
     for (int k = 1; k < 32; k <<= 1) {
         const int o = __shfl_up_sync(0xffffffffu, v, k);
         if (lane >= k) v += o;
     }
-    part[lane][g] = v - own;
-    if (lane == 31 && blockIdx.x * CHUNK_DIGITS + g < width)
-        total[blockIdx.x * CHUNK_DIGITS + g] = v;
+    part[lane][w] = v - own;
+    if (lane == 31 && blockIdx.x * CHUNK_DIGITS + w < width)
+        total[blockIdx.x * CHUNK_DIGITS + w] = v;
     __syncthreads();
-    if (d < width) {
-        int p = part[g][lane];
-#pragma unroll 8
-        for (int c = c0; c < c1; ++c) {
-            const long long i = (long long)c * width + d;
-            const int x = chunk_sum[i];
-            chunk_sum[i] = p;
-            p += x;
-        }
+    int p = part[g][j];
+#pragma unroll
+    for (int i = 0; i < SPAN; ++i) {
+        if (c0 + i < c1) chunk_sum[(long long)(c0 + i) * width + d] = p;
+        p += x[i];
     }
 }
 
@@ -551,7 +558,6 @@ __global__ void __launch_bounds__(THREADS, 3) bucket_scatter_kernel(
     const long long t0 = (long long)blockIdx.x * T;
     const int cnt = (int)min((long long)T, n - t0);
     const int mine = w * WSPAN + lane;       // this thread's entries: mine + 32 i
-    ptx::griddep_launch_dependents();
     for (int i = tid; i < NW * width / 8; i += THREADS)
         reinterpret_cast<uint4 *>(wcnt)[i] = make_uint4(0, 0, 0, 0);
     ptx::griddep_wait();
@@ -691,7 +697,7 @@ int count_digits(const int *key, long long n, int shift, int nb, const PassTable
                               t.chunk_base));
     const int width = table_width(nb);
     SBLAS_CUDA_TRY(launch_pdl(bucket_chunks_kernel,
-                              dim3((width + CHUNK_DIGITS - 1) / CHUNK_DIGITS), dim3(1024), 0,
+                              dim3((width + CHUNK_DIGITS - 1) / CHUNK_DIGITS), dim3(32 * CHUNK_DIGITS), 0,
                               stream, width, (int)t.chunks, t.chunk_base, t.total));
     return SBLAS_OK;
 }

@@ -142,15 +142,12 @@ __device__ __forceinline__ double2 ldg_x2(const double2 *p, uint64_t policy)
 }
 
 // Programmatic dependent launch.  A kernel launched with programmatic
-// stream serialisation may start before the previous kernel of its stream
-// has finished; griddep_wait() then blocks until that kernel has completed
-// and its writes are visible (a no-op without such a launch).
-// griddep_launch_dependents() lets the next kernel start early.
+// stream serialisation may start when the last CTA of the previous kernel of
+// its stream has exited, before that kernel has been flushed and retired;
+// griddep_wait() then blocks until it has completed and its writes are visible
+// (a no-op without such a launch).  No kernel here lets its successor start
+// earlier than that: see tile_spmv_kernel and bucket_sort.cuh.
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void griddep_launch_dependents()
-{
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
 
 }  // namespace ptx
 }  // namespace sblas

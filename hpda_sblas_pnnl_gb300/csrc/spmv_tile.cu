@@ -850,7 +850,7 @@ __global__ void __launch_bounds__(CTA_THREADS, min_ctas<SIGMA, VK>())
     // launched right behind the tile partition (or the fix-up of the product
     // before) with programmatic stream serialisation, which saves the launch
     // latency between them.  No kernel of this chain lets its successor start
-    // early (griddep_launch_dependents): the waiting CTAs then take registers
+    // early (griddepcontrol.launch_dependents): its waiting CTAs then take registers
     // and thread slots beside the ones that run, and tile CTAs are placed
     // around them unevenly.  With early starts / without: analysed product,
     // banded 6.4M nonzeros FP32 26.9 / 24.3 us, 17M power-law 87.0 / 85.0;
