@@ -30,8 +30,8 @@
 // digits.  Equal digits by ballots rather than __match_any_sync, which takes a
 // warp's distinct values one after another: 312 -> 289 us in a copy of the
 // pass; CTAs of 512 threads (twice the warp-private tables): 326 us.
-// CSC to CSR, 20M entries, 1M rows: 890 -> 608 us; one product of a CSC matrix
-// with 4.5M entries: 275 -> 171 us.
+// CSC to CSR, 20M entries, 1M rows: 890 -> 523 us; one product of a CSC matrix
+// with 4.5M entries: 275 -> 155 us.
 #pragma once
 
 #include <atomic>
@@ -49,7 +49,7 @@ namespace bsort {
 // could be moved ahead of the wait for that kernel.  (None of them lets its
 // successor start before its last CTA exits: with early starts the waiting CTAs
 // take slots and shared memory from the running ones, 20M entries 608 -> 617
-// us, 4.5M 144 -> 148, small sorts the same.)
+// us, 4.5M 144 -> 148, small sorts the same; taken before the prefetches.)
 // internal linkage: every translation unit that includes this header gets its
 // own copy of the kernels (no relocatable device code)
 namespace {
@@ -565,6 +565,21 @@ __global__ void __launch_bounds__(THREADS, 3) bucket_scatter_kernel(
 #pragma unroll
     for (int i = 0; i < ITER; ++i)
         key[i] = mine + 32 * i < cnt ? *(op.key_in + t0 + mine + 32 * i) : 0;
+    // The arrays that are moved after the keys on their way to L2 from the start,
+    // one prefetch per 64 bytes: a tile's phases wait for their loads one after
+    // another, and holding the values in registers meanwhile spills (20M
+    // entries 594 -> 691 us).  Prefetched: 594 -> 523, 4.5M entries 142 -> 128 (one
+    // prefetch per 128 bytes 562 / 137; a tile of the next wave as well 547 / 133).
+    constexpr int PF = 64;
+    if (op.d_out)
+#pragma unroll
+        for (int e = tid * (PF / 8); e < T; e += THREADS * (PF / 8))
+            if (e < cnt) ptx::prefetch_l2(op.d_in + t0 + e);
+    if constexpr (!SEG)
+        if (op.a_out)
+#pragma unroll
+            for (int e = tid * (PF / 4); e < T; e += THREADS * (PF / 4))
+                if (e < cnt) ptx::prefetch_l2(op.a_in + t0 + e);
     __syncthreads();
     unsigned short *mycnt = wcnt + w * width;
     int slot[ITER];
