@@ -536,7 +536,7 @@ def run_powerlaw_forms_extra(dev, stream, args, timed, threads, pk, forms):
                                    "staging indices, once per pattern; bound_values_us: "
                                    "executor with values kept in row order (sblas_csc_bind_values); "
                                    "one_shot_us: sblas_dcscmv (inspector without staging, "
-                                   "values gathered directly, tile kernel)"}
+                                   "values carried by its sort, tile kernel)"}
     del colptr, rowidx, cval
     torch.cuda.empty_cache()
     row = synth.csr_to_coo_rows(a)

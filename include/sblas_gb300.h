@@ -159,8 +159,7 @@ SBLAS_API int sblas_dcoomv(int m, int n, long long nnz, double alpha, const doub
                  void *stream);
 
 /* CSC -> CSR on the device (stable; columns ascending inside each row): a
- * least-significant-digit bucket sort by row, 8-bit digits (three passes
- * up to 16M rows).
+ * least-significant-digit bucket sort by row (two passes up to 4M rows).
  * work: sblas_csc_to_csr_workspace_bytes(m, n, nnz) bytes. */
 SBLAS_API size_t sblas_csc_to_csr_workspace_bytes(int m, int n, long long nnz);
 SBLAS_API int sblas_csc_to_csr(int m, int n, long long nnz, const double *csc_val,
@@ -173,9 +172,9 @@ SBLAS_API int sblas_csc_to_csr(int m, int n, long long nnz, const double *csc_va
  * (src/dspmv_mgpu_baseline_csc.cu:131-135 runs it as a transposed csrmv).
  * Inspector: a stable bucket sort of the entries by row gives A's row-ordered
  * structure and the permutation to it (sblas_csc_analyse, into `work`;
- * patterns above 2^20 entries also get staging indices); executor: the
- * values moved into row order (through L2-resident staging buckets after
- * sblas_csc_analyse; one direct gather in sblas_dcscmv) and the CSR tile
+ * patterns above 2^25 entries also get staging indices); executor: the
+ * values moved into row order (one direct gather, or through L2-resident
+ * staging buckets; the sort of sblas_dcscmv carries them) and the CSR tile
  * kernel (sblas_dcscmv_analysed, with the same work, colptr/rowidx
  * unchanged; val == NULL: the values last bound with sblas_csc_bind_values):
  * no atomics, bit-reproducible.  sblas_dcscmv runs both.  Rows need not be
