@@ -417,7 +417,8 @@ inline int exclusive_scan(const int *in, int *out, long long n, void *tmp, int *
 
 // ---- stable scatter ---------------------------------------------------------
 // What a pass moves: the keys and up to two ints and one double per entry.
-// An output that is null is not carried.
+// An output that is null is not carried; scatter_pass_iter refuses an output
+// without its input, so the kernel tests outputs only.
 //   SEG   a is not read but is the segment (column of CSC, row of CSR) of the
 //         entry in ptr[0 .. nseg]
 //   IDX   b is not read but is the entry's own position
@@ -740,6 +741,11 @@ int scatter_pass_iter(const Arrays &op, long long n, int shift, int nb, void *wo
     if (n <= 0) return SBLAS_OK;
     if (nb < 1 || nb > MAXB || (nb & (nb - 1)) != 0) {
         set_error(SBLAS_ERR_ARG, "bucket pass: %d buckets", nb);
+        return SBLAS_ERR_ARG;
+    }
+    if (op.key_in == nullptr || (op.d_out && !op.d_in) || (op.a_out && !(SEG ? op.ptr : op.a_in)) ||
+        (op.b_out && !IDX && !op.b_in)) {
+        set_error(SBLAS_ERR_ARG, "sort: null device pointer");
         return SBLAS_ERR_ARG;
     }
     const PassTables t = pass_tables(n, nb, ITER, work);

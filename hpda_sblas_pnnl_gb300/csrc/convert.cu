@@ -273,10 +273,13 @@ int launch_csc_to_csr(int m, int n, long long nnz, const double *csc_val, const 
     ArraySet out;
     out.key = reinterpret_cast<int *>(w);   // the rows, sorted: the row pointer's source
     out.a = csr_col;
-    out.d = csr_val;
+    out.d = csc_val != nullptr ? csr_val : nullptr;
     const int rc = lsd_sort<true, false>(first, nnz, m, out, w + al256(4 * (size_t)nnz),
                             work_bytes - al256(4 * (size_t)nnz), stream);
     if (rc != SBLAS_OK) return rc;
+    // no values (a pattern): those of the CSR matrix are zeros
+    if (csc_val == nullptr && csr_val != nullptr)
+        SBLAS_CUDA_TRY(cudaMemsetAsync(csr_val, 0, sizeof(double) * (size_t)nnz, stream));
     return launch_coo_rows_to_rowptr(m, nnz, out.key, csr_rowptr, stream);
 }
 

@@ -160,6 +160,7 @@ SBLAS_API int sblas_dcoomv(int m, int n, long long nnz, double alpha, const doub
 
 /* CSC -> CSR on the device (stable; columns ascending inside each row): a
  * least-significant-digit bucket sort by row (two passes up to 4M rows).
+ * csc_val == NULL (a pattern): csr_val, where given, is filled with zeros.
  * work: sblas_csc_to_csr_workspace_bytes(m, n, nnz) bytes. */
 SBLAS_API size_t sblas_csc_to_csr_workspace_bytes(int m, int n, long long nnz);
 SBLAS_API int sblas_csc_to_csr(int m, int n, long long nnz, const double *csc_val,

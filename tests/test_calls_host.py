@@ -1,0 +1,29 @@
+"""Calls of the C entry points and of the Python layer that are decided on the
+host, before anything is launched (no GPU)."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+
+SBLAS_ERR_ARG, SBLAS_ERR_CUDA = -1, -3
+
+
+def _addr(a):
+    return C.c_void_p(a.ctypes.data)
+
+
+@pytest.mark.parametrize("missing", ["colptr", "rowidx"])
+def test_sort_refuses_an_output_without_its_input(sblas_lib, missing):
+    """A null array that a pass of the sort would read is an argument error, not
+    a launch (host arrays stand in for device arrays: nothing reads them)."""
+    m, n, nnz = 50, 40, 300
+    ints = {k: np.zeros(nnz + m + n + 2, np.int32) for k in ("colptr", "rowidx", "rp", "col")}
+    val = np.zeros(nnz)
+    wb = sblas_lib.sblas_csc_to_csr_workspace_bytes(m, n, nnz)
+    work = np.zeros(wb + 256, np.uint8)
+    ptr = {k: None if k == missing else _addr(a) for k, a in ints.items()}
+    for given in (None, _addr(val)):
+        rc = sblas_lib.sblas_csc_to_csr(m, n, nnz, given, ptr["colptr"], ptr["rowidx"], _addr(val),
+                                        ptr["rp"], ptr["col"], _addr(work), wb, None)
+        assert rc == SBLAS_ERR_ARG
