@@ -154,6 +154,10 @@ int launch_coo_rows_to_rowptr(int m, long long nnz, const int *coo_row, int *row
 
 namespace {
 
+// The passes read their tables 16 bytes at a time and the caller's workspace
+// may start anywhere: the scratch begins at the next boundary (total has room).
+constexpr size_t kSortAlign = 16;
+
 // Buffers of one stable least-significant-digit sort of n entries: the pass
 // scratch (digit-count table, scan sums) and, for two passes or more, one or
 // two sets of intermediate arrays (key, a, b, d as present).
@@ -172,7 +176,7 @@ LsdLayout lsd_layout(long long n, long long key_bound, bool has_a, bool has_b, b
     L.pass = al256(bsort::pass_work_bytes(n > 0 ? n : 1, 1 << plan.width));
     L.set = al256(4 * nn) + (has_a ? al256(4 * nn) : 0) + (has_b ? al256(4 * nn) : 0) +
             (has_d ? al256(8 * nn) : 0);
-    L.total = L.pass + (size_t)(L.passes >= 3 ? 2 : (L.passes == 2 ? 1 : 0)) * L.set;
+    L.total = kSortAlign + L.pass + (size_t)(L.passes >= 3 ? 2 : (L.passes == 2 ? 1 : 0)) * L.set;
     return L;
 }
 
@@ -214,7 +218,8 @@ int lsd_sort(const bsort::Arrays &first, long long n, long long key_bound, const
         set_error(SBLAS_ERR_ARG, "sort workspace too small (%zu < %zu)", work_bytes, L.total);
         return SBLAS_ERR_ARG;
     }
-    unsigned char *w = static_cast<unsigned char *>(work);
+    unsigned char *w = reinterpret_cast<unsigned char *>(
+        (reinterpret_cast<uintptr_t>(work) + kSortAlign - 1) & ~uintptr_t(kSortAlign - 1));
     ArraySet tmp[2] = {array_set(w + L.pass, n, has_a, has_b, has_d),
                        array_set(w + L.pass + L.set, n, has_a, has_b, has_d)};
     const int nb = 1 << L.width;

@@ -43,3 +43,44 @@ def test_csc_to_csr_of_a_pattern(sblas_lib, cuda, nnz, m):
                           np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=m))]))
     assert np.array_equal(c.cpu().numpy(), cols[order])
     assert not v.any()
+
+
+@pytest.mark.parametrize("nnz", [1, 5000, (1 << 19) + 1, (1 << 22) + 1])
+@pytest.mark.parametrize("m", [900, 60_000, 5_000_000])
+@pytest.mark.parametrize("offset", [0, 4, 8, 20])
+def test_sort_workspace_at_any_alignment(sblas_lib, cuda, nnz, m, offset):
+    """The sorts ask for bytes of workspace, not for an alignment: one, two and
+    three passes with the workspace `offset` bytes into an allocation, and
+    nothing written past the bytes that were asked for."""
+    n = 3000
+    colptr, rows, cols = csc_pattern(m, n, nnz, nnz)
+    val = np.random.default_rng(1).standard_normal(nnz)
+    order = np.argsort(rows, kind="stable")
+    rowptr = np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=m))])
+    cp, ri, v = (torch.from_numpy(a).to(cuda) for a in (colptr, rows, val))
+    rp = torch.empty(m + 1, dtype=torch.int32, device=cuda)
+    c, perm = (torch.empty(nnz, dtype=torch.int32, device=cuda) for _ in range(2))
+    out = torch.empty(nnz, dtype=torch.float64, device=cuda)
+    stream = C.c_void_p(torch.cuda.current_stream(cuda).cuda_stream)
+
+    def work(size):
+        t = torch.full((size + offset + 64,), 0x5A, dtype=torch.uint8, device=cuda)
+        return t, t.data_ptr() + offset, t[offset + size:]
+
+    wb = sblas_lib.sblas_csc_to_csr_workspace_bytes(m, n, nnz)
+    keep, w, rest = work(wb)
+    assert sblas_lib.sblas_csc_to_csr(m, n, nnz, v.data_ptr(), cp.data_ptr(), ri.data_ptr(),
+                                      out.data_ptr(), rp.data_ptr(), c.data_ptr(), w, wb, stream) == 0
+    assert np.array_equal(rp.cpu().numpy(), rowptr)
+    assert np.array_equal(c.cpu().numpy(), cols[order])
+    assert np.array_equal(out.cpu().numpy(), val[order])
+    assert bool((rest == 0x5A).all())
+    # the same arrays as a CSR matrix of n rows: its transpose
+    wb = sblas_lib.sblas_csr_transpose_workspace_bytes(n, m, nnz)
+    keep, w, rest = work(wb)
+    assert sblas_lib.sblas_csr_transpose(n, m, nnz, cp.data_ptr(), ri.data_ptr(), rp.data_ptr(),
+                                         c.data_ptr(), perm.data_ptr(), w, wb, stream) == 0
+    assert np.array_equal(rp.cpu().numpy(), rowptr)
+    assert np.array_equal(c.cpu().numpy(), cols[order])
+    assert np.array_equal(perm.cpu().numpy(), order)
+    assert bool((rest == 0x5A).all())
