@@ -460,16 +460,18 @@ __device__ __forceinline__ void tile_segments(const int *ptr, int nseg, long lon
     // segments holding entries t0 and tl: lo + (probes <= the entry) * step
     int lo = 0, hi = nseg, lo2 = 0, hi2 = nseg;
     while (hi - lo > 1 || hi2 - lo2 > 1) {   // the answers are in [lo, hi), [lo2, hi2)
-        const int st = (hi - lo + THREADS) / (THREADS + 1);
-        const int st2 = (hi2 - lo2 + THREADS) / (THREADS + 1);
+        // rounded up; written so that no step of it leaves 32 bits at 2^31 - 1
+        // segments
+        const int st = (hi - lo - 1) / (THREADS + 1) + 1;
+        const int st2 = (hi2 - lo2 - 1) / (THREADS + 1) + 1;
         const long long p = lo + (long long)(tid + 1) * st, p2 = lo2 + (long long)(tid + 1) * st2;
         const bool le = p < hi && (long long)*(ptr + p) <= t0;
         const bool le2 = p2 < hi2 && (long long)*(ptr + p2) <= tl;
         const int c = __syncthreads_count(le), c2 = __syncthreads_count(le2);
         lo += c * st;
-        hi = min(hi, lo + st);
+        hi = lo + min(hi - lo, st);
         lo2 += c2 * st2;
-        hi2 = min(hi2, lo2 + st2);
+        hi2 = lo2 + min(hi2 - lo2, st2);
     }
     __syncthreads();   // seg is cleared
     for (long long s = (long long)lo + 1 + tid; s <= lo2; s += THREADS) {

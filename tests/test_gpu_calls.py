@@ -84,3 +84,21 @@ def test_sort_workspace_at_any_alignment(sblas_lib, cuda, nnz, m, offset):
     assert np.array_equal(c.cpu().numpy(), cols[order])
     assert np.array_equal(perm.cpu().numpy(), order)
     assert bool((rest == 0x5A).all())
+
+
+def test_sort_with_the_most_columns(sblas_lib, cuda):
+    """2^31 - 1 columns with entries in the last of them: the search for an entry's
+    column stays in 32 bits."""
+    from hpda_sblas_pnnl_gb300 import ops
+    m, n = 7, (1 << 31) - 1
+    at = [n - 90_000, n - 70_000, n - 514, n - 300, n - 258, n - 257, n - 2, n - 1]
+    colptr = torch.zeros(n + 1, dtype=torch.int32, device=cuda)
+    for c in at:
+        colptr[c + 1:] += 1
+    rows = torch.tensor([3, 0, 3, 6, 6, 1, 0, 3], dtype=torch.int32, device=cuda)
+    val = torch.arange(8, dtype=torch.float64, device=cuda)
+    rp, c, v = ops.csc_to_csr(m, n, colptr, rows, val)
+    order = np.argsort(rows.cpu().numpy(), kind="stable")
+    assert c.cpu().tolist() == [at[i] for i in order]
+    assert v.cpu().tolist() == [float(i) for i in order]
+    assert rp.cpu().tolist() == [0, 2, 3, 3, 6, 6, 6, 8]
