@@ -65,7 +65,6 @@ DeviceContext *device_context()
         if (cudaEventCreate(&e) != cudaSuccess) return nullptr;
     for (auto &e : c.chunk_ev)
         if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return nullptr;
-    if (cudaMallocHost(&c.host_word, sizeof(int)) != cudaSuccess) return nullptr;
     c.num_sms = sms;
     c.stream = st;
     c.copy_stream = cst;

@@ -266,6 +266,7 @@ spmv_ret run_host(Call c)
     }
     spmv_ret ret = zero_ret();
     if (c.m == 0) return ret;
+    if (!ctx->host_word) DROPIN_CUDA(cudaMallocHost(&ctx->host_word, sizeof(int)));
     if (c.fmt == Fmt::CSR && c.kernel != 1 && c.n > 0 && c.row_lo == 0 && c.row_hi == c.m) {
         const int K = host_chunks(c.nnz, c.nnz > 0 && is_pinned(c.val));
         if (K > 0) return run_host_pipelined(c, ctx, K);

@@ -196,9 +196,10 @@ struct DeviceContext {
     cudaStream_t copy_stream = nullptr;   // host -> device copies overlapping the kernels
     cudaEvent_t ev[6] = {};
     cudaEvent_t chunk_ev[kPipeChunks + 2] = {};  // copies done (row pointer, x and y, each chunk)
-    int *host_word = nullptr;   // pinned: a launch's status word
+    int *host_word = nullptr;   // pinned: a launch's status word (made by the first host-array call)
 };
-// Returns the context of the current device (created on first use).
+// Returns the context of the current device (created on first use, which may be
+// inside a stream capture: nothing in it allocates memory).
 DeviceContext *device_context();
 
 // Grow-only device scratch buffers owned by the context (slot 0..15).

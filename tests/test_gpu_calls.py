@@ -3,6 +3,9 @@ left out, empty matrices, workspaces at any alignment, one call after another
 on the same workspace.  Whole numbers and moved values equal, FP64 sums
 within 1e-12 relative L2."""
 import ctypes as C
+import subprocess
+import sys
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -102,3 +105,29 @@ def test_sort_with_the_most_columns(sblas_lib, cuda):
     assert c.cpu().tolist() == [at[i] for i in order]
     assert v.cpu().tolist() == [float(i) for i in order]
     assert rp.cpu().tolist() == [0, 2, 3, 3, 6, 6, 6, 8]
+
+
+def test_first_call_inside_a_capture(sblas_lib, cuda):
+    """The library's first call in a process may be one that is captured: a
+    caller's workspace, nothing allocated, nothing run before."""
+    code = """
+import torch
+from hpda_sblas_pnnl_gb300 import ops
+m, per = 20_000, 20
+col = torch.arange(m * per, device="cuda", dtype=torch.int32) % m
+rp = (torch.arange(m + 1, device="cuda") * per).int()
+val = torch.ones(m * per, dtype=torch.float64, device="cuda")
+x = torch.ones(m, dtype=torch.float64, device="cuda")
+y = torch.zeros(m, dtype=torch.float64, device="cuda")
+work = torch.empty(ops.workspace_bytes(m * per), dtype=torch.uint8, device="cuda")
+torch.cuda.synchronize()
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g):
+    ops.csrmv(rp, col, val, x, y, work=work)
+g.replay()
+torch.cuda.synchronize()
+assert bool((y == per).all())
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300,
+                       cwd=Path(__file__).resolve().parents[1])
+    assert r.returncode == 0, r.stderr[-2000:]
