@@ -334,6 +334,7 @@ int sblas_dcscmv(int m, int n, long long nnz, double alpha, const double *val, c
         return SBLAS_ERR_ARG;
     }
     const size_t need = cscmv_workspace_bytes(m, n, nnz);
+    const bool own_work = work != nullptr;
     if (work == nullptr) {
         work = device_scratch(14, need);
         work_bytes = need;
@@ -342,7 +343,7 @@ int sblas_dcscmv(int m, int n, long long nnz, double alpha, const double *val, c
             return SBLAS_ERR_ALLOC;
         }
     }
-    return launch_cscmv(m, n, nnz, alpha, val, colptr, rowidx, x, beta, y, work, work_bytes,
+    return launch_cscmv(m, n, nnz, alpha, val, colptr, rowidx, x, beta, y, work, work_bytes, own_work,
                         static_cast<cudaStream_t>(stream));
 }
 

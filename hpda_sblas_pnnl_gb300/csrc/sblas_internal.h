@@ -172,9 +172,10 @@ int launch_csc_bind_values(int m, int n, long long nnz, const double *val, void 
 int launch_cscmv_analysed(int m, int n, long long nnz, double alpha, const double *val,
                           const double *x, double beta, double *y, void *work,
                           size_t work_bytes, cudaStream_t stream);
+// keep_analysis: the work of a pattern of up to 2^20 entries holds an analysis afterwards
 int launch_cscmv(int m, int n, long long nnz, double alpha, const double *val,
                  const int *colptr, const int *rowidx, const double *x, double beta, double *y,
-                 void *work, size_t work_bytes, cudaStream_t stream);
+                 void *work, size_t work_bytes, bool keep_analysis, cudaStream_t stream);
 void *csc_tile_workspace(void *work, int m, int n, long long nnz);
 // Stable sort of COO entries by keys in [0, key_bound), carrying the other
 // index and the value (bucket_sort.cuh passes).  Workspace:

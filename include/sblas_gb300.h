@@ -178,8 +178,10 @@ SBLAS_API int sblas_csc_to_csr(int m, int n, long long nnz, const double *csc_va
  * staging buckets; the sort of sblas_dcscmv carries them) and the CSR tile
  * kernel (sblas_dcscmv_analysed, with the same work, colptr/rowidx
  * unchanged; val == NULL: the values last bound with sblas_csc_bind_values):
- * no atomics, bit-reproducible.  sblas_dcscmv runs both.  Rows need not be
- * sorted inside a column.  work: sblas_cscmv_workspace_bytes(m, n, nnz)
+ * no atomics, bit-reproducible.  sblas_dcscmv runs both; in a caller's `work`
+ * it leaves an analysis as sblas_csc_analyse does for patterns of up to 2^20
+ * entries (above, run sblas_csc_analyse).  Rows need not be sorted inside a
+ * column.  work: sblas_cscmv_workspace_bytes(m, n, nnz)
  * bytes, 256-byte aligned (sblas_dcscmv: or NULL for a library-owned
  * buffer).  A bounded wait that gave up is reported by sblas_stream_status. */
 SBLAS_API size_t sblas_cscmv_workspace_bytes(int m, int n, long long nnz);

@@ -131,3 +131,33 @@ assert bool((y == per).all())
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300,
                        cwd=Path(__file__).resolve().parents[1])
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("nnz", [1, 3000, 200_000, 1 << 20])
+def test_one_shot_csc_product_leaves_an_analysis(sblas_lib, cuda, nnz):
+    """sblas_dcscmv in the caller's workspace, then products with other values
+    of the pattern, and with bound ones, from the same workspace."""
+    from hpda_sblas_pnnl_gb300 import _lib, ops
+    m, n = 70_000, 9000
+    colptr, rows, cols = csc_pattern(m, n, nnz, nnz)
+    rng = np.random.default_rng(2)
+    x, y0 = rng.standard_normal(n), rng.standard_normal(m)
+    cp, ri, xd = (torch.from_numpy(a).to(cuda) for a in (colptr, rows, x))
+    wb = sblas_lib.sblas_cscmv_workspace_bytes(m, n, nnz)
+    work = torch.full((wb,), 0xFF, dtype=torch.uint8, device=cuda)
+    stream = C.c_void_p(torch.cuda.current_stream(cuda).cuda_stream)
+    for step in range(3):
+        val = rng.standard_normal(nnz)
+        v, y = torch.from_numpy(val).to(cuda), torch.from_numpy(y0).to(cuda)
+        if step == 0:
+            ops.cscmv(cp, ri, v, xd, y, 1.5, -0.5, work=work)
+        else:
+            if step == 2:
+                _lib.check(sblas_lib.sblas_csc_bind_values(m, n, nnz, v.data_ptr(), work.data_ptr(),
+                                                           wb, stream))
+            _lib.check(sblas_lib.sblas_dcscmv_analysed(
+                m, n, nnz, 1.5, v.data_ptr() if step == 1 else None, xd.data_ptr(), -0.5,
+                y.data_ptr(), work.data_ptr(), wb, stream))
+        ref = -0.5 * y0
+        np.add.at(ref, rows, 1.5 * val * x[cols])
+        assert rel_l2(y.cpu().numpy(), ref) <= RTOL_L2, step
