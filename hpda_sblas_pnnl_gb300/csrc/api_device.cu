@@ -460,7 +460,7 @@ int sblas_dspmspv(int kernel, int m, int n, long long nnz, double alpha, const d
         return SBLAS_ERR_ARG;
     }
     if (kernel == 1) {
-        if (val == nullptr) {
+        if (val == nullptr && nnz > 0) {   // an empty FP64 array may be null
             set_error(SBLAS_ERR_UNSUPPORTED, "kernel 1 takes FP64 values only");
             return SBLAS_ERR_UNSUPPORTED;
         }

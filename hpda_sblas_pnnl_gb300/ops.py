@@ -594,6 +594,8 @@ def spmspv(rowptr: torch.Tensor, col: torch.Tensor, val: torch.Tensor | None, x:
     _require_dtype("y", y, torch.float64)
     if y.numel() != m:
         raise ValueError("shape mismatch")
+    if val is None and kernel == KERNEL_ROWSPLIT and m > 0:   # refused without nonzeros too
+        raise _lib.SblasError(-7, "kernel 1 takes FP64 values only")
     lib = _lib.load()
     wb = lib.sblas_dspmspv_workspace_bytes(m, x.numel(), nnz)
     work = torch.empty(wb, dtype=torch.uint8, device=dev) if wb else None

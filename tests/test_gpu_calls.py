@@ -161,3 +161,23 @@ def test_one_shot_csc_product_leaves_an_analysis(sblas_lib, cuda, nnz):
         ref = -0.5 * y0
         np.add.at(ref, rows, 1.5 * val * x[cols])
         assert rel_l2(y.cpu().numpy(), ref) <= RTOL_L2, step
+
+
+@pytest.mark.parametrize("kernel", [1, 2, 3])
+def test_spmspv_of_an_empty_matrix(sblas_lib, cuda, kernel):
+    """No nonzeros: y = beta * y for every kernel that takes the form of the
+    values; kernel 1 refuses a pattern, empty or not."""
+    from hpda_sblas_pnnl_gb300 import _lib, ops
+    rp = torch.zeros(6, dtype=torch.int32, device=cuda)
+    col = torch.zeros(0, dtype=torch.int32, device=cuda)
+    val = torch.zeros(0, dtype=torch.float64, device=cuda)
+    x = torch.ones(3, dtype=torch.float64, device=cuda)
+    y = torch.full((5,), 3.0, dtype=torch.float64, device=cuda)
+    ops.spmspv(rp, col, val, x, y, 1.0, 0.5, kernel=kernel)
+    assert y.tolist() == [1.5] * 5
+    if kernel == 1:
+        with pytest.raises(_lib.SblasError):
+            ops.spmspv(rp, col, None, x, y, 1.0, 0.5, kernel=kernel)
+    else:
+        ops.spmspv(rp, col, None, x, y, 1.0, 0.0, kernel=kernel)
+        assert y.tolist() == [0.0] * 5
