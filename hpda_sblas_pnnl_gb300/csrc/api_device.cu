@@ -184,7 +184,8 @@ static int csrmv(int kernel, int m, int n, long long nnz, double alpha, const vo
             return SBLAS_ERR_UNSUPPORTED;
         }
         if (nnz > 0 && small_spmv_fits(m, n, nnz, false))
-            return launch_small_spmv(m, alpha, val, val_kind, rowptr, col, x, beta, y, nullptr, st);
+            return launch_small_spmv(m, nnz, alpha, val, val_kind, rowptr, col, x, beta, y, nullptr,
+                                     st);
         return launch_rowsplit_spmv(m, n, nnz, alpha, static_cast<const double *>(val), rowptr,
                                     col, x, beta, y, st);
     }
@@ -465,8 +466,8 @@ int sblas_dspmspv(int kernel, int m, int n, long long nnz, double alpha, const d
             return SBLAS_ERR_UNSUPPORTED;
         }
         if (nnz > 0 && small_spmv_fits(m, n, nnz, false))
-            return launch_small_spmv(m, alpha, val, VAL_F64, rowptr, col, x, beta, y, nullptr, st,
-                                     true);
+            return launch_small_spmv(m, nnz, alpha, val, VAL_F64, rowptr, col, x, beta, y, nullptr,
+                                     st, true);
         return launch_rowsplit_spmv(m, n, nnz, alpha, val, rowptr, col, x, beta, y, st, true);
     }
     const int sigma = default_sigma_for(m, nnz);

@@ -114,11 +114,12 @@ int launch_tile_analyse(int m, long long nnz, const int *rowptr, int sigma, void
 
 // Small matrices (spmv_small.cu): one launch, no workspace.  Callers that
 // leave the tile shape to the library take it where small_spmv_fits.
-// status: cleared, or null.  skip_zero_x as in launch_tile_spmv.
+// nnz: entries of val and col (none past them is read).  status: cleared, or
+// null.  skip_zero_x as in launch_tile_spmv.
 bool small_spmv_fits(int m, int n, long long nnz, bool analysed);
-int launch_small_spmv(int m, double alpha, const void *val, int val_kind, const int *rowptr,
-                      const int *col, const double *x, double beta, double *y, int *status,
-                      cudaStream_t stream, bool skip_zero_x = false);
+int launch_small_spmv(int m, long long nnz, double alpha, const void *val, int val_kind,
+                      const int *rowptr, const int *col, const double *x, double beta, double *y,
+                      int *status, cudaStream_t stream, bool skip_zero_x = false);
 int small_spmv_preload_f64();
 
 // Row-split kernel (one sub-warp per row; kernel version 1).

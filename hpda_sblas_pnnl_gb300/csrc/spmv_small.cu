@@ -24,6 +24,7 @@ constexpr int WARP_ROW = 512;              // longest row of a warp
 
 struct SmallArgs {
     int m;
+    int nnz;            // entries of val and col
     double alpha, beta;
     const void *val;
     const int *rowptr;
@@ -99,10 +100,11 @@ __global__ void __launch_bounds__(THREADS) small_spmv_kernel(const SmallArgs a, 
         const long long row = (step + g) * gridDim.x + blockIdx.x;
         const bool in = g < rows && row < a.m;
         const int r = (int)row;
+        // a row's end past the entries there are is cut off, as the tiles do
         int b = 0, e = 0;
         if (in) {
-            b = a.rowptr[r];
-            e = a.rowptr[r + 1];
+            b = max(a.rowptr[r], 0);
+            e = min(a.rowptr[r + 1], a.nnz);
         }
         const bool mine = in && e - b <= LANE_ROW;
         if (in && !mine && l == 0) long_row[atomicAdd(&nlong, 1)] = r;
@@ -116,7 +118,7 @@ __global__ void __launch_bounds__(THREADS) small_spmv_kernel(const SmallArgs a, 
         const int n = nlong;
         for (int i = 0; i < n; ++i) {   // the list's order does not matter: a row is one sum
             const int q = long_row[i];
-            const int qb = a.rowptr[q], qe = a.rowptr[q + 1];
+            const int qb = max(a.rowptr[q], 0), qe = min(a.rowptr[q + 1], a.nnz);
             if (qe - qb <= WARP_ROW) {
                 if (i % WARPS != w) continue;
                 double t = dot<VK, SKIP, 8>(a, qb, qe, lane, 32);
@@ -179,12 +181,12 @@ bool small_spmv_fits(int m, int n, long long nnz, bool analysed)
     return nnz <= (analysed && nnz > 8LL * m ? 32768 : 131072);
 }
 
-int launch_small_spmv(int m, double alpha, const void *val, int val_kind, const int *rowptr,
-                      const int *col, const double *x, double beta, double *y, int *status,
-                      cudaStream_t stream, bool skip_zero_x)
+int launch_small_spmv(int m, long long nnz, double alpha, const void *val, int val_kind,
+                      const int *rowptr, const int *col, const double *x, double beta, double *y,
+                      int *status, cudaStream_t stream, bool skip_zero_x)
 {
     if (m <= 0) return SBLAS_OK;
-    const SmallArgs a{m, alpha, beta, val, rowptr, col, x, y, status};
+    const SmallArgs a{m, (int)nnz, alpha, beta, val, rowptr, col, x, y, status};
     if (skip_zero_x) {
         if (val_kind == VAL_F64) return launch<VAL_F64, true>(a, stream);
         if (val_kind == VAL_PATTERN) return launch<VAL_PATTERN, true>(a, stream);

@@ -1442,7 +1442,7 @@ int launch_tile_spmv(int m, int n, long long nnz, double alpha, const void *val,
     if (m <= 0) return SBLAS_OK;
     if (nnz <= 0) return launch_scale_y(m, beta, y, stream);
     if (auto_shape && small_spmv_fits(m, n, nnz, analysed))
-        return launch_small_spmv(m, alpha, val, val_kind, rowptr, col, x, beta, y,
+        return launch_small_spmv(m, nnz, alpha, val, val_kind, rowptr, col, x, beta, y,
                                  reset_status ? status_in(work) : nullptr, stream, skip_zero_x);
     if (tile_shape_index(sigma) < 0) {
         set_error(SBLAS_ERR_UNSUPPORTED, "sigma %d is not a compiled tile shape", sigma);

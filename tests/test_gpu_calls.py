@@ -181,3 +181,30 @@ def test_spmspv_of_an_empty_matrix(sblas_lib, cuda, kernel):
     else:
         ops.spmspv(rp, col, None, x, y, 1.0, 0.0, kernel=kernel)
         assert y.tolist() == [0.0] * 5
+
+
+@pytest.mark.parametrize("lengths", [[3, 4], [5, 0, 700, 3] * 40, [60, 600, 7] * 9, [4] * 3000],
+                         ids=lambda v: f"{len(v)}x{max(v)}")
+@pytest.mark.parametrize("short", [1, 5, 300])
+def test_small_matrix_reads_no_entry_past_its_arrays(sblas_lib, cuda, lengths, short):
+    """A row pointer that says more than col and val hold (they are views of
+    longer arrays with NaN behind): the entries that are there, for lanes, warps
+    and the CTA, with and without zeros of x left out."""
+    from hpda_sblas_pnnl_gb300 import ops
+    rng = np.random.default_rng(short)
+    n, m = 400, len(lengths)
+    rp = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
+    have = max(int(rp[-1]) - short, 1)
+    col = rng.integers(0, n, rp[-1]).astype(np.int32)
+    val, x = rng.standard_normal(rp[-1]), rng.standard_normal(n)
+    ref = np.zeros(m)
+    rows = np.repeat(np.arange(m), lengths)
+    np.add.at(ref, rows[:have], val[:have] * x[col[:have]])
+    val[have:] = np.nan
+    trp, tcol, tval, tx = (torch.from_numpy(a).to(cuda) for a in (rp, col, val, x))
+    tcol, tval = tcol[:have], tval[:have]
+    y = torch.empty(m, dtype=torch.float64, device=cuda)
+    for kernel in (2, 3):
+        assert rel_l2(ops.csrmv(trp, tcol, tval, tx, y, kernel=kernel).cpu().numpy(), ref) <= RTOL_L2
+        assert rel_l2(ops.spmspv(trp, tcol, tval, tx, y, kernel=kernel).cpu().numpy(), ref) <= RTOL_L2
+    assert rel_l2(ops.CsrPlan(trp, tcol, tval, n=n)(tx, y).cpu().numpy(), ref) <= RTOL_L2
