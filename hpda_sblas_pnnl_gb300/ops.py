@@ -607,12 +607,14 @@ def spmspv(rowptr: torch.Tensor, col: torch.Tensor, val: torch.Tensor | None, x:
     return y
 
 
-def check_device(device: torch.device | None = None, clear: bool = True) -> None:
-    """Waits for the current stream of `device`, then raises SblasError
+def check_device(device: torch.device | str | int | None = None, clear: bool = True) -> None:
+    """Waits for the current stream of `device` (None: the current device), then raises SblasError
     (SBLAS_ERR_TIMEOUT) if a tile kernel launched on that device gave up one
     of its bounded waits since the last check: the y of that launch is only
     partly written.  clear=True resets the device's sticky word."""
-    dev = torch.device("cuda", torch.cuda.current_device()) if device is None else device
+    dev = torch.device("cuda" if device is None else device)
+    if dev.index is None:
+        dev = torch.device(dev.type, torch.cuda.current_device())
     with _guard(dev):
         rc = _lib.load().sblas_stream_status(_stream_ptr(dev), 1 if clear else 0)
     _lib.check(rc)
