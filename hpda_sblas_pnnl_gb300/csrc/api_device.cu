@@ -63,8 +63,10 @@ DeviceContext *device_context()
     if (cudaStreamCreateWithFlags(&cst, cudaStreamNonBlocking) != cudaSuccess) return nullptr;
     for (auto &e : c.ev)
         if (cudaEventCreate(&e) != cudaSuccess) return nullptr;
+    for (auto &e : c.run_ev)
+        if (cudaEventCreate(&e) != cudaSuccess) return nullptr;
     for (auto &e : c.chunk_ev)
-        if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return nullptr;
+        if (cudaEventCreate(&e) != cudaSuccess) return nullptr;
     c.num_sms = sms;
     c.stream = st;
     c.copy_stream = cst;

@@ -4,10 +4,11 @@
 // replaces: partition (trivial for one part), host->device copies, one
 // device kernel, device->host copy of y, merge.  Timing fields of spmv_ret
 // follow the reference: comm_time = host->device copies (CUDA events,
-// src/dspmv_mgpu_baseline.cu:114-120), comp_time = SpMV kernel (events,
-// :124-130), part_time = partition / format work, merg_time = device->host
-// copy and host merge (wall clock, :156-165), numa_part_time = 0 (no NUMA
-// staging copy on a one-GPU, one-NUMA-node process).
+// src/dspmv_mgpu_baseline.cu:114-120), comp_time = SpMV kernels (events,
+// :124-130; the tile partition among them), part_time = format work (COO and
+// CSC calls), merg_time = device->host copy after the last kernel (events, or
+// the wall clock as at :156-165 in calls that run in chunks), numa_part_time = 0
+// (no NUMA staging copy on a one-GPU, one-NUMA-node process).
 #include <sys/time.h>
 
 #include <algorithm>
@@ -199,15 +200,17 @@ spmv_ret run_host_pipelined(const Call &c, DeviceContext *ctx, int K)
         set_error(SBLAS_ERR_ALLOC, "%s: device allocation failed", c.name);
         return failed();
     }
-    cudaEvent_t e0 = ctx->ev[0], e1 = ctx->ev[1], e2 = ctx->ev[2], e3 = ctx->ev[3];
+    cudaEvent_t e0 = ctx->ev[0];
+    int runs = 0;   // chunk_ev and run_ev recorded: the partition, then each chunk
     const bool y_pinned = is_pinned(c.y);
     // ---- the row pointer and its partition, then x (and y when it is read)
     DROPIN_CUDA(cudaEventRecord(e0, cs));
+    const double t0_wall = wall();
     DROPIN_CUDA(cudaMemcpyAsync(d_ptr, c.ptr, sizeof(int) * (size_t)(m + 1), cudaMemcpyHostToDevice, cs));
     DROPIN_CUDA(cudaEventRecord(ctx->chunk_ev[0], cs));
     DROPIN_CUDA(cudaStreamWaitEvent(ks, ctx->chunk_ev[0], 0));
-    DROPIN_CUDA(cudaEventRecord(e2, ks));
     if (launch_tile_analyse(m, nnz, d_ptr, sigma, w, ks) != SBLAS_OK) return failed();
+    DROPIN_CUDA(cudaEventRecord(ctx->run_ev[runs++], ks));
     DROPIN_CUDA(cudaMemcpyAsync(d_x, c.x, sizeof(double) * (size_t)n, cudaMemcpyHostToDevice, cs));
     if (need_y_in)
         DROPIN_CUDA(cudaMemcpyAsync(d_y, c.y, sizeof(double) * (size_t)m, cudaMemcpyHostToDevice, cs));
@@ -222,12 +225,12 @@ spmv_ret run_host_pipelined(const Call &c, DeviceContext *ctx, int K)
                                     cudaMemcpyHostToDevice, cs));
         DROPIN_CUDA(cudaMemcpyAsync(d_idx + lo, c.idx + lo, sizeof(int) * (size_t)(hi - lo),
                                     cudaMemcpyHostToDevice, cs));
-        DROPIN_CUDA(cudaEventRecord(ctx->chunk_ev[1 + k], cs));
-        if (t1 == ntiles) DROPIN_CUDA(cudaEventRecord(e1, cs));
-        DROPIN_CUDA(cudaStreamWaitEvent(ks, ctx->chunk_ev[1 + k], 0));
+        DROPIN_CUDA(cudaEventRecord(ctx->chunk_ev[runs], cs));
+        DROPIN_CUDA(cudaStreamWaitEvent(ks, ctx->chunk_ev[runs], 0));
         if (launch_tile_range(m, n, nnz, c.alpha, d_val, SBLAS_VAL_F64, d_ptr, d_idx, d_x, beta_eff,
                               d_y, sigma, w, ks, t0, t1, t0 == 0) != SBLAS_OK)
             return failed();
+        DROPIN_CUDA(cudaEventRecord(ctx->run_ev[runs++], ks));
         if (!y_pinned) continue;
         // the rows that end before tile t1 are complete
         const int end = t1 == ntiles ? m
@@ -239,19 +242,26 @@ spmv_ret run_host_pipelined(const Call &c, DeviceContext *ctx, int K)
         row = std::max(row, end);
     }
     if (tile_workspace_status(w, ctx->host_word, ks) != SBLAS_OK) return failed();
-    DROPIN_CUDA(cudaEventRecord(e3, ks));
-    const double tm = wall();
     if (!y_pinned)
         DROPIN_CUDA(cudaMemcpyAsync(c.y, d_y, sizeof(double) * (size_t)m, cudaMemcpyDeviceToHost, ks));
     DROPIN_CUDA(cudaStreamSynchronize(ks));
+    const double wall_s = wall() - t0_wall;
     if (!launches_completed(c, ctx)) return failed();
+    // A stretch of kernels runs from when its copies are there and the stretch
+    // before is done to its own event: what it waits for stays out of comp_time.
     spmv_ret ret = zero_ret();
-    float t_comm = 0.f, t_comp = 0.f;
-    DROPIN_CUDA(cudaEventElapsedTime(&t_comm, e0, e1));
-    DROPIN_CUDA(cudaEventElapsedTime(&t_comp, e2, e3));
-    ret.comm_time = t_comm * 1e-3;   // host-to-device copies (overlapping the kernels)
-    ret.comp_time = t_comp * 1e-3;   // kernels (and copies of y back) from the partition on
-    ret.merg_time = wall() - tm;
+    float copied = 0.f, done = 0.f;   // ms from e0
+    for (int i = 0; i < runs; ++i) {
+        const float before = done;
+        DROPIN_CUDA(cudaEventElapsedTime(&copied, e0, ctx->chunk_ev[i]));
+        DROPIN_CUDA(cudaEventElapsedTime(&done, e0, ctx->run_ev[i]));
+        ret.comp_time += std::max(0.f, done - std::max(copied, before)) * 1e-3;
+    }
+    ret.comm_time = copied * 1e-3;   // host-to-device copies
+    // y's copy after the last kernel, by the host's clock: an event after a copy
+    // to pageable memory, which is over when it returns, is one more wait for the
+    // GPU (13 us of a call of 640 us)
+    ret.merg_time = std::max(0.0, wall_s - done * 1e-3);
     return ret;
 }
 

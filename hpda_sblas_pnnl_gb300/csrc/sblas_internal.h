@@ -197,7 +197,10 @@ struct DeviceContext {
     cudaStream_t stream = nullptr;
     cudaStream_t copy_stream = nullptr;   // host -> device copies overlapping the kernels
     cudaEvent_t ev[6] = {};
-    cudaEvent_t chunk_ev[kPipeChunks + 2] = {};  // copies done (row pointer, x and y, each chunk)
+    // of a chunked host call: copies done (row pointer, each chunk) and kernels
+    // done (partition, each chunk)
+    cudaEvent_t chunk_ev[kPipeChunks + 1] = {};
+    cudaEvent_t run_ev[kPipeChunks + 1] = {};
     int *host_word = nullptr;   // pinned: a launch's status word (made by the first host-array call)
 };
 // Returns the context of the current device (created on first use, which may be

@@ -5,6 +5,7 @@ within 1e-12 relative L2."""
 import ctypes as C
 import subprocess
 import sys
+import time
 from pathlib import Path
 
 import numpy as np
@@ -208,3 +209,31 @@ def test_small_matrix_reads_no_entry_past_its_arrays(sblas_lib, cuda, lengths, s
         assert rel_l2(ops.csrmv(trp, tcol, tval, tx, y, kernel=kernel).cpu().numpy(), ref) <= RTOL_L2
         assert rel_l2(ops.spmspv(trp, tcol, tval, tx, y, kernel=kernel).cpu().numpy(), ref) <= RTOL_L2
     assert rel_l2(ops.CsrPlan(trp, tcol, tval, n=n)(tx, y).cpu().numpy(), ref) <= RTOL_L2
+
+
+@pytest.mark.parametrize("pinned", [False, True])
+@pytest.mark.parametrize("nnz", [1 << 18, 1 << 21, (1 << 22) - 1, 1 << 22, (1 << 24) + 5])
+def test_host_call_times_are_of_what_they_say(sblas_lib, cuda, pinned, nnz):
+    """comp_time is the kernels' time, with and without chunks: the copies that
+    they wait for stay out.  A product reads its 12 bytes per nonzero at several
+    TB/s, the copies move them at a few hundred GB/s at most: far below half
+    of the copies' time (from 2^21 nonzeros on, where launches count little);
+    and the parts of a call are not longer than the call."""
+    from hpda_sblas_pnnl_gb300 import api
+    rng = np.random.default_rng(nnz)
+    m, n = nnz // 20, 40_000
+    rp = np.minimum(np.arange(m + 1, dtype=np.int64) * 20, nnz).astype(np.int32)
+    rp[-1] = nnz
+    col = rng.integers(0, n, nnz).astype(np.int32)
+    val, x, y = rng.standard_normal(nnz), rng.standard_normal(n), np.zeros(m)
+    if pinned:
+        keep = [torch.from_numpy(a).pin_memory() for a in (val, rp, col, x, y)]
+        val, rp, col, x, y = (t.numpy() for t in keep)
+    for _ in range(3):
+        t0 = time.perf_counter()
+        r = api.spMV_mgpu_v1(m, n, nnz, 1.0, val, rp, col, x, 0.0, y)
+        wall = time.perf_counter() - t0
+    assert 0 < r.comp_time and 0 < r.comm_time and 0 <= r.merg_time and r.part_time >= 0
+    assert max(r.comp_time, r.comm_time, r.merg_time) <= wall
+    if nnz >= 1 << 21:
+        assert r.comp_time <= 0.5 * r.comm_time, (r.comp_time, r.comm_time)
