@@ -60,7 +60,10 @@ __global__ void batch_partition_kernel(const Mat *mats, int nmat, int *unit_mat,
 }
 
 bool k_compiled(int k) { return k == 1 || k == 2 || k == 4 || k == 8 || k == 16; }
-bool s_compiled(int s) { return s == 4 || s == 8 || s == 16 || s == 32; }
+bool s_compiled(int k, int s)
+{
+    return s == 4 || s == 8 || s == 16 || s == 32 || (k >= 8 && (s == 1 || s == 2));
+}
 
 // Nonzeros per lane when the caller leaves the choice to the plan (s = 0), by
 // k and the nonzeros of the whole batch.  Two costs meet: a unit is walked
@@ -262,8 +265,8 @@ int sblas_batch_plan_create(int nmat, const sblas_batch_matrix *mats, int k, int
         set_error(SBLAS_ERR_UNSUPPORTED, "k = %d not compiled (1, 2, 4, 8, 16)", k);
         return SBLAS_ERR_UNSUPPORTED;
     }
-    if (s != 0 && !s_compiled(s)) {
-        set_error(SBLAS_ERR_UNSUPPORTED, "s = %d not compiled (4, 8, 16, 32)", s);
+    if (s != 0 && !s_compiled(k, s)) {
+        set_error(SBLAS_ERR_UNSUPPORTED, "s = %d not compiled (4, 8, 16, 32; 1 and 2 for k >= 8)", s);
         return SBLAS_ERR_UNSUPPORTED;
     }
     if (val_kind < SBLAS_VAL_F64 || val_kind > SBLAS_VAL_PATTERN) {

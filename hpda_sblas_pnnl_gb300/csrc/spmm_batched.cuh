@@ -1135,7 +1135,7 @@ cudaError_t dispatch_k(Op op, int S, int VK, const Args *a, int nunits, int grid
                                  : shape_grid<K, SS, VV>(nunits, grid_out);
 #define SBLAS_BATCH_S(SS)                                                                \
     SBLAS_BATCH_SHAPE(SS, VAL_F64) SBLAS_BATCH_SHAPE(SS, VAL_F32) SBLAS_BATCH_SHAPE(SS, VAL_PATTERN)
-    if constexpr (use_vec<K>()) {   // chosen by the plan for small matrices only
+    if constexpr (use_vec<K>()) {   // for small matrices
         SBLAS_BATCH_S(1)
         SBLAS_BATCH_S(2)
     }

@@ -1,7 +1,8 @@
 """Autotuner: picks tile shapes by timing the compiled candidates on the
 caller's own matrices (CUDA events on the current stream, after a warm-up).
 
-  batch_s     nonzeros per lane (s) of the batched SpMM for a batch and k
+  batch_s     nonzeros per lane (s) of the batched SpMM for a batch and k, of
+              every compiled shape (candidates: some of them)
   spmm_s      the same for one matrix with k right-hand sides (ops.SpmmPlan)
   tile_sigma  nonzeros per thread (sigma) of the single-matrix tile kernel
 
@@ -35,7 +36,11 @@ def _time_ms(fn, reps: int) -> float:
     return statistics.median(ts)
 
 
-def batch_s(matrices, xs, k: int, candidates=(4, 8, 16, 32), reps: int = 5):
+def _shapes(k: int) -> tuple:
+    return (1, 2, 4, 8, 16, 32) if k >= 8 else (4, 8, 16, 32)
+
+
+def batch_s(matrices, xs, k: int, candidates=None, reps: int = 5):
     """Best s for ops.BatchPlan(matrices, xs, ys, k); returns (s, {s: ms})."""
     key = ("batch", k, tuple((rp.numel() - 1, x.shape[0], c.numel(), ops._val_kind(v))
                              for (rp, c, v), x in zip(matrices, xs)))
@@ -44,7 +49,7 @@ def batch_s(matrices, xs, k: int, candidates=(4, 8, 16, 32), reps: int = 5):
     ys = [torch.empty((rp.numel() - 1, k) if k > 1 else (rp.numel() - 1,), dtype=torch.float64,
                       device=x.device) for (rp, _, _), x in zip(matrices, xs)]
     times = {}
-    for s in candidates:
+    for s in candidates or _shapes(k):
         plan = ops.BatchPlan(matrices, xs, ys, k, s=s)
         times[s] = _time_ms(plan, reps)
         plan.close()
@@ -54,7 +59,7 @@ def batch_s(matrices, xs, k: int, candidates=(4, 8, 16, 32), reps: int = 5):
 
 
 def spmm_s(rowptr: torch.Tensor, col: torch.Tensor, val: torch.Tensor | None, n: int, k: int,
-           candidates=(4, 8, 16, 32), reps: int = 5, row_ids: torch.Tensor | None = None,
+           candidates=None, reps: int = 5, row_ids: torch.Tensor | None = None,
            m_out: int | None = None, val_perm: torch.Tensor | None = None):
     """Best s for ops.SpmmPlan(rowptr, col, val, n, k); returns (s, {s: ms}).
     Times Y = A X on a scratch X of ones (the schedule does not depend on
@@ -67,7 +72,7 @@ def spmm_s(rowptr: torch.Tensor, col: torch.Tensor, val: torch.Tensor | None, n:
     x = torch.ones((n, k) if k > 1 else (n,), dtype=torch.float64, device=dev)
     y = torch.empty((m, k) if k > 1 else (m,), dtype=torch.float64, device=dev)
     times = {}
-    for s in candidates:
+    for s in candidates or _shapes(k):
         plan = ops.SpmmPlan(rowptr, col, val, n=n, k=k, s=s, row_ids=row_ids, m_out=m_out,
                             val_perm=val_perm)
         times[s] = _time_ms(lambda: plan(x, y), reps)

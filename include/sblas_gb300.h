@@ -213,8 +213,8 @@ SBLAS_API int sblas_coo_rows_to_rowptr(int m, long long nnz, const int *coo_row,
  * X_i: n_i x k, row-major, row stride ldx >= k (the k values of one row
  * contiguous); Y_i: m_i x k, row-major, row stride ldy >= k.  For k >= 2, x
  * and y must be 16-byte aligned and ldx, ldy even.  k in {1, 2, 4, 8, 16};
- * s in {4, 8, 16, 32} (0: picked by the plan from k and the batch's nonzeros;
- * sblas_batch_plan_info tells). */
+ * s in {4, 8, 16, 32}, for k >= 8 also {1, 2} (0: picked by the plan from k and
+ * the batch's nonzeros; sblas_batch_plan_info tells). */
 typedef struct sblas_batch_matrix {
     int m;
     int n;
@@ -241,7 +241,8 @@ typedef struct sblas_batch_matrix {
 
 typedef struct sblas_batch_plan sblas_batch_plan;
 
-/* Default nonzeros per lane for k right-hand sides (0 if k not compiled). */
+/* Nonzeros per lane for k right-hand sides where nothing is known of the
+ * matrices (0 if k not compiled); a plan made with s = 0 goes by their size. */
 SBLAS_API int sblas_batch_default_s(int k);
 /* Analysis: copies the descriptors to the device, computes the unit
  * partition and the persistent grid.  Allocates the plan's device memory

@@ -237,3 +237,47 @@ def test_host_call_times_are_of_what_they_say(sblas_lib, cuda, pinned, nnz):
     assert max(r.comp_time, r.comm_time, r.merg_time) <= wall
     if nnz >= 1 << 21:
         assert r.comp_time <= 0.5 * r.comm_time, (r.comp_time, r.comm_time)
+
+
+@pytest.mark.parametrize("k", [1, 2, 4, 8, 16])
+@pytest.mark.parametrize("s", [1, 2])
+@pytest.mark.parametrize("vals", ["f64", "f32"])
+def test_short_units_by_request(sblas_lib, cuda, k, s, vals):
+    """s = 1 and 2, which a plan picks for small matrices at k >= 8: rows at the
+    lengths of a unit and of the fix-up's runs, many rows in a unit, empty
+    rows; product, values' adjoint, and a plan made again from what it
+    reports.  Refused at smaller k, where they are not compiled."""
+    from hpda_sblas_pnnl_gb300 import _lib, ops
+    from oracle import oracle as O
+    unit = 32 * s
+    lengths = ([0, 1, unit - 1, 0, 0, unit, unit + 1] + [1] * (2 * unit + 3) + [0] * 40 + [2, 0] * unit +
+               [33 * unit, 7, 32 * unit - 7, 31 * unit, 3, 300 * unit + 5, 0])
+    n, m = 700, len(lengths)
+    rng = np.random.default_rng(k + s)
+    rp = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
+    col = rng.integers(0, n, rp[-1]).astype(np.int32)
+    val = rng.standard_normal(rp[-1])
+    trp, tcol, tval = (torch.from_numpy(a).to(cuda) for a in (rp, col, val))
+    if vals == "f32":
+        tval = tval.float()
+        val = tval.double().cpu().numpy()
+    if k < 8:
+        with pytest.raises(_lib.SblasError):
+            ops.SpmmPlan(trp, tcol, tval, n=n, k=k, s=s)
+        return
+    x, y0 = rng.standard_normal((n, k)), rng.standard_normal((m, k))
+    tx = torch.from_numpy(x).to(cuda)
+    plan = ops.SpmmPlan(trp, tcol, tval, n=n, k=k, s=s)
+    y = torch.from_numpy(y0).to(cuda)
+    plan(tx, y, 1.5, -0.5)
+    assert rel_l2(y.cpu().numpy(), O.csr_spmm(m, n, rp, col, val, x, y0.copy(), 1.5, -0.5)) <= RTOL_L2
+    dval = torch.empty_like(tval)
+    plan.sddmm(y, tx, dval)
+    ref = O.csr_sddmm(m, n, rp, col, y.cpu().numpy(), x)
+    assert rel_l2(dval.double().cpu().numpy(), ref) <= (RTOL_L2 if vals == "f64" else 2.0 ** -24)
+    # what a plan picks for a small matrix can be asked for
+    small = [torch.from_numpy(a).to(cuda) for a in (rp[:40] * 1, col, val)]
+    small[1], small[2] = small[1][:rp[39]].contiguous(), small[2][:rp[39]].contiguous()
+    picked = ops.SpmmPlan(*small, n=n, k=k).s
+    assert picked == 1
+    assert ops.SpmmPlan(*small, n=n, k=k, s=picked).s == picked
