@@ -185,7 +185,7 @@ static int csrmv(int kernel, int m, int n, long long nnz, double alpha, const vo
             set_error(SBLAS_ERR_UNSUPPORTED, "kernel 1 takes FP64 values only");
             return SBLAS_ERR_UNSUPPORTED;
         }
-        if (nnz > 0 && small_spmv_fits(m, n, nnz, false))
+        if (nnz > 0 && small_beats_rowsplit(m, n, nnz))
             return launch_small_spmv(m, nnz, alpha, val, val_kind, rowptr, col, x, beta, y, nullptr,
                                      st);
         return launch_rowsplit_spmv(m, n, nnz, alpha, static_cast<const double *>(val), rowptr,
@@ -467,7 +467,7 @@ int sblas_dspmspv(int kernel, int m, int n, long long nnz, double alpha, const d
             set_error(SBLAS_ERR_UNSUPPORTED, "kernel 1 takes FP64 values only");
             return SBLAS_ERR_UNSUPPORTED;
         }
-        if (nnz > 0 && small_spmv_fits(m, n, nnz, false))
+        if (nnz > 0 && small_beats_rowsplit(m, n, nnz))
             return launch_small_spmv(m, nnz, alpha, val, VAL_F64, rowptr, col, x, beta, y, nullptr,
                                      st, true);
         return launch_rowsplit_spmv(m, n, nnz, alpha, val, rowptr, col, x, beta, y, st, true);

@@ -117,6 +117,7 @@ int launch_tile_analyse(int m, long long nnz, const int *rowptr, int sigma, void
 // nnz: entries of val and col (none past them is read).  status: cleared, or
 // null.  skip_zero_x as in launch_tile_spmv.
 bool small_spmv_fits(int m, int n, long long nnz, bool analysed);
+bool small_beats_rowsplit(int m, int n, long long nnz);   // kernel 1
 int launch_small_spmv(int m, long long nnz, double alpha, const void *val, int val_kind,
                       const int *rowptr, const int *col, const double *x, double beta, double *y,
                       int *status, cudaStream_t stream, bool skip_zero_x = false);

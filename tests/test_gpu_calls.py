@@ -281,3 +281,57 @@ def test_short_units_by_request(sblas_lib, cuda, k, s, vals):
     picked = ops.SpmmPlan(*small, n=n, k=k).s
     assert picked == 1
     assert ops.SpmmPlan(*small, n=n, k=k, s=picked).s == picked
+
+
+def test_kernel_1_on_many_almost_empty_rows(sblas_lib, cuda):
+    """4M rows, 100K nonzeros: kernel 1 streams the row pointer and y (12 bytes
+    per row, 7 us at the memory's rate) and is not held up row by row."""
+    from hpda_sblas_pnnl_gb300 import ops
+    m, n, nnz = 4_000_000, 20_000, 100_000
+    rng = np.random.default_rng(1)
+    rows = np.sort(rng.integers(0, m, nnz))
+    rp = np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=m))]).astype(np.int32)
+    col, val, x = rng.integers(0, n, nnz).astype(np.int32), rng.standard_normal(nnz), rng.standard_normal(n)
+    ref = np.zeros(m)
+    np.add.at(ref, rows, val * x[col])
+    trp, tcol, tval, tx = (torch.from_numpy(a).to(cuda) for a in (rp, col, val, x))
+    y = torch.empty(m, dtype=torch.float64, device=cuda)
+    for call in (ops.csrmv, ops.spmspv):
+        best = 1e9
+        for _ in range(10):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            call(trp, tcol, tval, tx, y, kernel=1)
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b) * 1e3)
+        assert rel_l2(y.cpu().numpy(), ref) <= RTOL_L2
+        assert best <= 20 * 12 * m / 6.8e12 * 1e6, best
+
+
+@pytest.mark.parametrize("m", [4864, 4865, 78_000])
+def test_small_matrix_over_several_steps_of_the_grid(sblas_lib, cuda, m):
+    """More rows than one step of the grid covers, with rows for a warp and for
+    the CTA in the first and in later steps; kernel 1 on both sides of its rule."""
+    from hpda_sblas_pnnl_gb300 import ops
+    rng = np.random.default_rng(m)
+    lengths = rng.integers(0, 2, m)
+    for i, r in enumerate(rng.choice(m, 40, replace=False)):
+        lengths[r] = (65, 512, 513, 900)[i % 4]
+    lengths[-1], lengths[-2] = 700, 100
+    n = 3000
+    rp = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
+    nnz = int(rp[-1])
+    assert nnz <= 131_072
+    col, val = rng.integers(0, n, nnz).astype(np.int32), rng.standard_normal(nnz)
+    x, y0 = rng.standard_normal(n), rng.standard_normal(m)
+    ref = -0.5 * y0
+    np.add.at(ref, np.repeat(np.arange(m), lengths), 1.5 * val * x[col])
+    trp, tcol, tval, tx = (torch.from_numpy(a).to(cuda) for a in (rp, col, val, x))
+    for kernel in (1, 2, 3):
+        for call in (ops.csrmv, ops.spmspv):
+            y = torch.from_numpy(y0).to(cuda)
+            call(trp, tcol, tval, tx, y, 1.5, -0.5, kernel=kernel)
+            assert rel_l2(y.cpu().numpy(), ref) <= RTOL_L2, (kernel, call)
+    y = torch.from_numpy(y0).to(cuda)
+    assert rel_l2(ops.CsrPlan(trp, tcol, tval, n=n)(tx, y, 1.5, -0.5).cpu().numpy(), ref) <= RTOL_L2
