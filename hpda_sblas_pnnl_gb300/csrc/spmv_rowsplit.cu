@@ -28,8 +28,14 @@ __global__ void __launch_bounds__(256) rowsplit_kernel(int m, double alpha, doub
         const int b = __ldg(rowptr + row), e = __ldg(rowptr + row + 1);
         double s = 0.0;
         for (int j = b + lane_g; j < e; j += G) {
-            const double xj = __ldg(x + __ldg(col + j));
-            if (!SKIP || xj != 0.0) s = fma(__ldg(val + j), xj, s);
+            // (one expression for both cost the plain product 20 %: one row of 16K among
+            // 19K rows, 216 -> 269 us; the value's load went behind x's)
+            if constexpr (SKIP) {
+                const double xj = __ldg(x + __ldg(col + j));
+                if (xj != 0.0) s = fma(__ldg(val + j), xj, s);
+            } else {
+                s = fma(__ldg(val + j), __ldg(x + __ldg(col + j)), s);
+            }
         }
 #pragma unroll
         for (int o = G / 2; o > 0; o >>= 1) s += __shfl_down_sync(mask, s, o, G);
