@@ -29,7 +29,7 @@ __global__ void __launch_bounds__(256) rowsplit_kernel(int m, double alpha, doub
         double s = 0.0;
         for (int j = b + lane_g; j < e; j += G) {
             // (one expression for both cost the plain product 20 %: one row of 16K among
-            // 19K rows, 216 -> 269 us; the value's load went behind x's)
+            // 19K rows, 216 -> 264 us; the value's load went behind x's)
             if constexpr (SKIP) {
                 const double xj = __ldg(x + __ldg(col + j));
                 if (xj != 0.0) s = fma(__ldg(val + j), xj, s);

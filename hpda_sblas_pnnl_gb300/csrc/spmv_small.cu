@@ -183,19 +183,21 @@ bool small_spmv_fits(int m, int n, long long nnz, bool analysed)
 
 // Against the row-split kernel (kernel 1), which reads the row pointer and
 // writes y in order and waits at no barrier, but walks a long row with the lanes
-// of a mean one: only where every row of the matrix is in flight at once, 32
-// rows per SM.  us per product, row split / here, 8K and 131K nonzeros, rows of
-// about one length, then drawn towards the first rows, then one of up to 16K:
-//      1216 rows   2.5 / 2.6   3.4 / 3.7     13 / 4.5   45 / 12      59 / 5.3  58 / 12
-//      4864        2.8 / 2.5   4.0 / 3.5     27 / 4.4   30 / 9      197 / 5.4  57 / 11
-//     19456        2.4 / 3.8   3.6 / 4.6     18 / 5.1   73 / 8      194 / 6.4 217 / 12
-//     38912        2.5 / 6.2   3.4 / 7.0
+// of a mean one.  Up to 64 rows per SM, two CTAs, even rows lose half a
+// microsecond at most and uneven ones gain up to 400.  us per product, row split
+// / here, 8K and 131K nonzeros: rows of about one length, rows drawn towards the
+// first, one row of half the nonzeros (16K at most):
+//      1216 rows   2.5 / 2.6   3.4 / 3.7     13 / 4.5   45 / 12      59 / 5.3   58 / 12
+//      4864        2.8 / 2.5   4.0 / 3.5     27 / 4.4   30 / 9      197 / 5.4   57 / 11
+//      9728        2.5 / 2.9   3.8 / 3.7     22 / 4.5   47 / 8      216 / 5.7  111 / 11
+//     19456        2.4 / 3.8   3.6 / 4.6     18 / 5.1   73 / 8      194 / 6.4  217 / 12
+//     38912        2.5 / 6.2   3.4 / 7.0     15 / 6.7  111 / 8      213 / 7.5  408 / 13
 //       400K       5.3 / 44    6.4 / 49
 //        10M        90 / 964    91 / 999
-// (the tile path, which kernels 2 and 3 would take, at 10M rows: 27000 and 1700).
+// (The tile path, which kernels 2 and 3 would take, at 10M rows: 27000 and 1700.)
 bool small_beats_rowsplit(int m, int n, long long nnz)
 {
-    return m <= THREADS / LANES * device_num_sms() && small_spmv_fits(m, n, nnz, false);
+    return m <= 2 * (THREADS / LANES) * device_num_sms() && small_spmv_fits(m, n, nnz, false);
 }
 
 int launch_small_spmv(int m, long long nnz, double alpha, const void *val, int val_kind,

@@ -309,7 +309,7 @@ def test_kernel_1_on_many_almost_empty_rows(sblas_lib, cuda):
         assert best <= 20 * 12 * m / 6.8e12 * 1e6, best
 
 
-@pytest.mark.parametrize("m", [4864, 4865, 78_000])
+@pytest.mark.parametrize("m", [4865, 9728, 9729, 78_000])
 def test_small_matrix_over_several_steps_of_the_grid(sblas_lib, cuda, m):
     """More rows than one step of the grid covers, with rows for a warp and for
     the CTA in the first and in later steps; kernel 1 on both sides of its rule."""
