@@ -462,20 +462,26 @@ int sblas_dspmspv(int kernel, int m, int n, long long nnz, double alpha, const d
         set_error(SBLAS_ERR_ARG, "null device pointer");
         return SBLAS_ERR_ARG;
     }
+    const int sigma = default_sigma_for(m, nnz);
+    const size_t need = sblas_dspmspv_workspace_bytes(m, n, nnz);
+    const bool work_fits = work != nullptr && work_bytes >= need &&
+                           (reinterpret_cast<uintptr_t>(work) & 255) == 0;
     if (kernel == 1) {
         if (val == nullptr && nnz > 0) {   // an empty FP64 array may be null
             set_error(SBLAS_ERR_UNSUPPORTED, "kernel 1 takes FP64 values only");
             return SBLAS_ERR_UNSUPPORTED;
         }
-        if (nnz > 0 && small_beats_rowsplit(m, n, nnz))
+        // Rows split over lanes walk all of a long row to find the nonzeros that
+        // count, however few: filter and product took 334 us for 1M power-law
+        // rows and 1 % of x, the row-split kernel 582, the tiles 115 (3.3M
+        // nonzeros 139 / 165 / 46).  It is left for callers without a workspace
+        // and for many almost empty rows (spmv_small.cu; 2^18 rows 33 us there).
+        if (nnz > 0 && need == 0 && m <= (1 << 18))
             return launch_small_spmv(m, nnz, alpha, val, VAL_F64, rowptr, col, x, beta, y, nullptr,
                                      st, true);
-        return launch_rowsplit_spmv(m, n, nnz, alpha, val, rowptr, col, x, beta, y, st, true);
-    }
-    const int sigma = default_sigma_for(m, nnz);
-    const size_t need = sblas_dspmspv_workspace_bytes(m, n, nnz);
-    if (need > 0 && (work == nullptr || work_bytes < need ||
-                    (reinterpret_cast<uintptr_t>(work) & 255) != 0)) {
+        if (need == 0 || !work_fits)
+            return launch_rowsplit_spmv(m, n, nnz, alpha, val, rowptr, col, x, beta, y, st, true);
+    } else if (need > 0 && !work_fits) {
         set_error(SBLAS_ERR_ARG, "workspace needs %zu bytes at 256-byte alignment", need);
         return SBLAS_ERR_ARG;
     }

@@ -293,9 +293,9 @@ SBLAS_API int sblas_csr_filter_x(int m, long long nnz, const int *rowptr, const 
  * zero (spMspV_mgpu_v1 / _v2 on device arrays): the filter is taken inside
  * the product, so infinite or NaN values at zeros of x stay out of y.  val:
  * FP64, or NULL (pattern-only; kernels 2 and 3).  col and val may hold more
- * than rowptr[m] entries (nnz of them).  work: for kernels 2 and 3,
+ * than rowptr[m] entries (nnz of them).  work:
  * sblas_dspmspv_workspace_bytes(m, n, nnz) bytes, 256-byte aligned (0: none
- * needed).  No allocation, no synchronisation: can be captured in a graph. */
+ * needed); kernel 1 runs without it too, slower where rows are long.  No allocation, no synchronisation: can be captured in a graph. */
 SBLAS_API size_t sblas_dspmspv_workspace_bytes(int m, int n, long long nnz);
 SBLAS_API int sblas_dspmspv(int kernel, int m, int n, long long nnz, double alpha,
                             const double *val, const int *rowptr, const int *col,

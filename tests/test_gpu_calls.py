@@ -335,3 +335,46 @@ def test_small_matrix_over_several_steps_of_the_grid(sblas_lib, cuda, m):
             assert rel_l2(y.cpu().numpy(), ref) <= RTOL_L2, (kernel, call)
     y = torch.from_numpy(y0).to(cuda)
     assert rel_l2(ops.CsrPlan(trp, tcol, tval, n=n)(tx, y, 1.5, -0.5).cpu().numpy(), ref) <= RTOL_L2
+
+
+@pytest.mark.parametrize("m,nnz,long_row", [(3000, 600_000, 9000), (20_000, 100_000, 16_000),
+                                            (300_000, 100_000, 500), (200_000, 3_000_000, 11_000)])
+def test_spmspv_kernel_1_is_not_held_up_by_long_rows(sblas_lib, cuda, m, nnz, long_row):
+    """Kernel 1 with and without a workspace (infinite values at zeros of x left
+    out); through ops.spmspv, which passes one, it takes at most twice as long
+    as kernel 2."""
+    from hpda_sblas_pnnl_gb300 import _lib, ops
+    rng = np.random.default_rng(m)
+    n = 10_000
+    rows = rng.integers(0, m, nnz)
+    rows[:long_row] = m // 2
+    rows = np.sort(rows)
+    rp = np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=m))]).astype(np.int32)
+    col, val = rng.integers(0, n, nnz).astype(np.int32), rng.standard_normal(nnz)
+    x = rng.standard_normal(n) * (rng.random(n) < 0.02)
+    y0 = rng.standard_normal(m)
+    ref = -0.5 * y0
+    live = x[col] != 0.0
+    np.add.at(ref, rows[live], 1.5 * val[live] * x[col[live]])
+    val[~live] = np.inf
+    trp, tcol, tval, tx = (torch.from_numpy(a).to(cuda) for a in (rp, col, val, x))
+    y = torch.from_numpy(y0).to(cuda)
+    stream = C.c_void_p(torch.cuda.current_stream(cuda).cuda_stream)
+    _lib.check(sblas_lib.sblas_dspmspv(1, m, n, nnz, 1.5, tval.data_ptr(), trp.data_ptr(),
+                                       tcol.data_ptr(), tx.data_ptr(), -0.5, y.data_ptr(), None, 0,
+                                       stream))
+    assert rel_l2(y.cpu().numpy(), ref) <= RTOL_L2
+    best = {}
+    for kernel in (1, 2):
+        best[kernel] = 1e9
+        for _ in range(10):
+            y.copy_(torch.from_numpy(y0))
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            torch.cuda.synchronize()
+            a.record()
+            ops.spmspv(trp, tcol, tval, tx, y, 1.5, -0.5, kernel=kernel)
+            b.record()
+            b.synchronize()
+            best[kernel] = min(best[kernel], a.elapsed_time(b) * 1e3)
+        assert rel_l2(y.cpu().numpy(), ref) <= RTOL_L2, kernel
+    assert best[1] <= 2 * best[2], best
