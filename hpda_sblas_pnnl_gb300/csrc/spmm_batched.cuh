@@ -268,9 +268,15 @@ __device__ __forceinline__ void gather_row(const double *x, long long c, int ldx
 // 2.0e7 / 2.1e7 nonzeros (power-law / banded), S = 16, 1, 2, 3, 4 and 8 rows:
 // K = 2 169/164, 151/147, 168/162, 154/149, 164/150 us; K = 4 239/237,
 // 251/247, 240/231, 250/254, 246/220 us (80 nonzeros per row: 185, 193, 187, 196,
-// 195 us).
-template <int K>
-constexpr int prefetch_rows() { return K == 2 ? 2 : K == 4 ? 3 : 1; }
+// 195 us).  K = 2 with FP32 values and S = 16 lost by two (one row issued ahead of
+// the multiply-adds / 2 / 3 / 4 rows): 1.5e7 banded 109 / 124 / 104 / 122, 1.6e7
+// power-law 110 / 123 / 104 / 122, 2.0e6 banded 28 / 28 / 25 / 28; pattern-only the
+// same with 2 and 3, S = 8 better with 2.
+template <int K, int S, int VK>
+constexpr int prefetch_rows()
+{
+    return K == 2 ? (VK == VAL_F32 && S >= 16 ? 3 : 2) : K == 4 ? 3 : 1;
+}
 
 template <int K>
 __device__ __forceinline__ void store_row(double *dst, const double (&a)[K])
@@ -365,7 +371,7 @@ __global__ void __launch_bounds__(CTA) batch_spmm_kernel(const Args a)
         const int cnt = max(0, min(S, cntu - c0));
         const int s0 = U0 + c0, send = s0 + cnt;
         double xs[K == 1 ? S : 1];       // K == 1: every gather issued up front
-        constexpr int PF = prefetch_rows<K>();
+        constexpr int PF = prefetch_rows<K, S, VK>();
         double ahead[PF][K];             // K >= 2: PF rows of X ahead
         if (cnt > 0) {
             if constexpr (K == 1) {
