@@ -66,7 +66,7 @@ bool s_compiled(int k, int s)
 }
 
 // Nonzeros per lane when the caller leaves the choice to the plan (s = 0), by
-// k and the nonzeros of the whole batch.  Two costs meet: a unit is walked
+// k, the nonzeros and the rows of the whole batch.  Two costs meet: a unit is walked
 // serially (32 s nonzeros by one warp), so a small matrix wants many short
 // units to occupy the 152 SMs; and every unit pays its staging, row search,
 // carries and fix-up, so a large one wants long units, up to where the
@@ -98,13 +98,31 @@ bool s_compiled(int k, int s)
 // unit's staging waits for random sectors, and more and shorter units hide
 // that better (1M rows, 2.0e7 nonzeros, s = 8 against 16: k = 8 466/471
 // against 577/436 us, k = 16 720/748 against 792/700).
-int pick_s(int k, long long nnz, bool permuted_f64)
+// Short rows cost a unit as much as its nonzeros do, and a long unit's more than
+// fit the row buffer: 4.0e6 nonzeros in 3.0e6 rows, s = 4 / 8 / 16: k = 2 71 / 73 /
+// 99, k = 4 128 / 132 / 158, k = 16 213 / 224 / 243; three such matrices k = 8 383 /
+// 356 / 424, k = 16 589 / 566 / 657.  Rows longer than a unit gain from long ones
+// earlier: 9e5 nonzeros, 428 per row, s = 4 / 8: k = 8 34 / 28, k = 16 46 / 39.
+// Permuted FP64 values at k = 4: 5000 rows of 800, s = 8 / 16: 99 / 126 (50 per row
+// and a local permutation 270 / 221).  Pattern-only at k = 1, where a lane's gathers
+// are all it stages: 1.6e6 28 / 25, 1.5e7 77 / 70, 2.0e6 banded 20 / 21.
+// The units of one matrix with values may serve the values' adjoint too, which
+// takes less time in short units as long as there are few (6e5 nonzeros,
+// s = 8 / 16: k = 4 12 / 18 against 22 / 21 us for the product; k = 2, 1.6e6: 17 / 26
+// against 35 / 32); those of a batch, a transpose or a pattern serve products alone.
+int pick_s(int k, long long nnz, long long rows, int nmat, int val_kind, bool permuted)
 {
+    const bool permuted_f64 = permuted && val_kind == SBLAS_VAL_F64;
+    const bool products = nmat > 1 || permuted || val_kind == SBLAS_VAL_PATTERN;
+    const bool brief = nnz < 4 * rows, wide = nnz >= 16 * rows;
     if (k >= 8)
-        return nnz < (1 << 14) ? 1 : nnz < 200000 ? 2 : nnz < 1000000 ? 4
-               : nnz < 6000000 || permuted_f64 ? 8 : 16;
+        return nnz < (1 << 14) ? 1 : nnz < 200000 ? 2 : nnz < (wide ? 800000 : 1000000) ? 4
+               : nnz < 6000000 ? (brief && k == 16 ? 4 : 8) : permuted_f64 || brief ? 8 : 16;
     if (nnz < (1 << 14)) return 4;
-    return (k == 4 && nnz >= 400000) || (k == 2 && nnz >= 2000000) ? 16 : 8;
+    if (brief || (permuted_f64 && k == 4 && nnz >= 256 * rows)) return 8;
+    if (k == 4) return nnz >= (products ? 400000 : 1000000) ? 16 : 8;
+    if (k == 2) return nnz >= (products && !permuted_f64 ? 600000 : 2000000) ? 16 : 8;
+    return val_kind == SBLAS_VAL_PATTERN && nnz >= 1000000 ? 16 : 8;
 }
 
 bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -274,13 +292,14 @@ int sblas_batch_plan_create(int nmat, const sblas_batch_matrix *mats, int k, int
         return SBLAS_ERR_ARG;
     }
     if (s == 0) {
-        long long nnz = 0;
+        long long nnz = 0, rows = 0;
         bool permuted = false;
         for (int i = 0; i < nmat; ++i) {
             nnz += mats[i].nnz > 0 ? mats[i].nnz : 0;
+            rows += mats[i].m > 0 ? mats[i].m : 0;
             permuted |= mats[i].val_perm != nullptr;
         }
-        s = pick_s(k, nnz, permuted && val_kind == SBLAS_VAL_F64);
+        s = pick_s(k, nnz, rows, nmat, val_kind, permuted);
     }
     const long long unit = 32LL * s;
     std::vector<Mat> dm(nmat);

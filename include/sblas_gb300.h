@@ -214,7 +214,7 @@ SBLAS_API int sblas_coo_rows_to_rowptr(int m, long long nnz, const int *coo_row,
  * contiguous); Y_i: m_i x k, row-major, row stride ldy >= k.  For k >= 2, x
  * and y must be 16-byte aligned and ldx, ldy even.  k in {1, 2, 4, 8, 16};
  * s in {4, 8, 16, 32}, for k >= 8 also {1, 2} (0: picked by the plan from k and
- * the batch's nonzeros; sblas_batch_plan_info tells). */
+ * the batch's nonzeros and rows; sblas_batch_plan_info tells). */
 typedef struct sblas_batch_matrix {
     int m;
     int n;

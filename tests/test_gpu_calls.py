@@ -378,3 +378,40 @@ def test_spmspv_kernel_1_is_not_held_up_by_long_rows(sblas_lib, cuda, m, nnz, lo
             best[kernel] = min(best[kernel], a.elapsed_time(b) * 1e3)
         assert rel_l2(y.cpu().numpy(), ref) <= RTOL_L2, kernel
     assert best[1] <= 2 * best[2], best
+
+
+@pytest.mark.parametrize("k", [2, 4, 8, 16])
+@pytest.mark.parametrize("m,nnz", [(3_000_000, 4_000_000), (6_000_000, 7_000_000), (700, 300_000),
+                                   (2000, 900_000), (30_000, 1_200_000)])
+def test_plans_picked_for_short_and_long_rows(sblas_lib, cuda, k, m, nnz):
+    """s = 0 on matrices with about one nonzero per row, and with hundreds: one
+    matrix and a batch, product and values' adjoint, and no long units where
+    a unit would hold more rows than nonzeros fit."""
+    from hpda_sblas_pnnl_gb300 import ops
+    g = torch.Generator(device=cuda)
+    g.manual_seed(nnz + k)
+    n = 4000
+    rows = torch.sort(torch.randint(0, m, (nnz,), generator=g, device=cuda)).values
+    rp = torch.zeros(m + 1, dtype=torch.int32, device=cuda)
+    rp[1:] = torch.cumsum(torch.bincount(rows, minlength=m), 0).int()
+    col = torch.randint(0, n, (nnz,), generator=g, device=cuda, dtype=torch.int32)
+    val = torch.randn(nnz, generator=g, dtype=torch.float64, device=cuda)
+    x = torch.randn((n, k), generator=g, dtype=torch.float64, device=cuda)
+    y0 = torch.randn((m, k), generator=g, dtype=torch.float64, device=cuda)
+    ref = -0.5 * y0
+    ref.index_add_(0, rows, 1.5 * val[:, None] * x[col.long()])
+    plan = ops.SpmmPlan(rp, col, val, n=n, k=k)
+    y = y0.clone()
+    plan(x, y, 1.5, -0.5)
+    assert float((y - ref).norm() / ref.norm()) <= RTOL_L2
+    dval = torch.empty_like(val)
+    plan.sddmm(y0, x, dval)
+    dref = (y0[rows] * x[col.long()]).sum(1)
+    assert float((dval - dref).norm() / dref.norm()) <= RTOL_L2
+    ys = [y0.clone() for _ in range(2)]
+    batch = ops.BatchPlan([(rp, col, val)] * 2, [x] * 2, ys, k, alpha=1.5, beta=-0.5)
+    batch()
+    for y in ys:
+        assert float((y - ref).norm() / ref.norm()) <= RTOL_L2
+    if nnz < 4 * m:
+        assert plan.s <= 8 and batch.s <= 8
