@@ -183,9 +183,10 @@ def cscmv(colptr: torch.Tensor, rowidx: torch.Tensor, val: torch.Tensor, x: torc
           y: torch.Tensor, alpha: float = 1.0, beta: float = 0.0,
           work: torch.Tensor | None = None) -> torch.Tensor:
     """y = alpha*A*x + beta*y with A in CSC (sblas_dcscmv): the row-ordered
-    structure by a stable bucket sort (inspector), then the values gathered
-    into row order and the CSR tile kernel: atomic-free, bit-reproducible.
-    work: optional uint8 device buffer of cscmv_workspace_bytes(m, n, nnz)."""
+    structure and the values in that order by a stable bucket sort, then the
+    CSR tile kernel: atomic-free, bit-reproducible.  work: optional uint8
+    device buffer of cscmv_workspace_bytes(m, n, nnz); up to 2^20 entries it
+    then holds an analysis (the values are gathered by it)."""
     dev = _require_cuda(colptr, rowidx, val, x, y, work)
     for what, t, dt in (("colptr", colptr, torch.int32), ("rowidx", rowidx, torch.int32),
                         ("val", val, torch.float64), ("x", x, torch.float64),
@@ -211,8 +212,9 @@ class CscPlan:
     of patterns above 2^25 entries and the tile partition, held in the
     plan's workspace); each call runs only the executor
     (sblas_dcscmv_analysed: the values moved into row order and the tile
-    kernel), with the values, x and y given per call; bind() keeps one set
-    of values in row order (calls with val=None then skip the move)."""
+    kernel), with the values, x and y given per call; bind() puts a set of
+    values in row order (calls with val=None then skip the move).  There is
+    room for one set: a call with values of its own replaces it."""
 
     def __init__(self, m: int, colptr: torch.Tensor, rowidx: torch.Tensor):
         dev = _require_cuda(colptr, rowidx)
@@ -229,8 +231,9 @@ class CscPlan:
         _lib.check(rc)
 
     def bind(self, val: torch.Tensor) -> None:
-        """Keeps these values (CSC order) in row order inside the plan: calls
-        with val=None then use them and skip the per-call gather."""
+        """Puts these values (CSC order) in row order inside the plan: calls
+        with val=None then use them and skip the per-call gather, until a call
+        with values of its own puts those in their place."""
         if _require_cuda(val) != self.device:
             raise ValueError("val must be on the plan's device")
         _require_dtype("val", val, torch.float64)

@@ -177,7 +177,8 @@ SBLAS_API int sblas_csc_to_csr(int m, int n, long long nnz, const double *csc_va
  * values moved into row order (one direct gather, or through L2-resident
  * staging buckets; the sort of sblas_dcscmv carries them) and the CSR tile
  * kernel (sblas_dcscmv_analysed, with the same work, colptr/rowidx
- * unchanged; val == NULL: the values last bound with sblas_csc_bind_values):
+ * unchanged; val == NULL: the values that `work` holds in row order, which are
+ * those last given to sblas_csc_bind_values or to a product in this `work`):
  * no atomics, bit-reproducible.  sblas_dcscmv runs both; in a caller's `work`
  * it leaves an analysis as sblas_csc_analyse does for patterns of up to 2^20
  * entries (above, run sblas_csc_analyse).  Rows need not be sorted inside a
@@ -193,10 +194,11 @@ SBLAS_API int sblas_csc_analyse(int m, int n, long long nnz, const int *colptr,
 SBLAS_API int sblas_dcscmv_analysed(int m, int n, long long nnz, double alpha, const double *val,
                                     const double *x, double beta, double *y, void *work,
                                     size_t work_bytes, void *stream);
-/* Keeps `val` (CSC order) in row order inside the analysis in `work`;
+/* Puts `val` (CSC order) in row order inside the analysis in `work`;
  * sblas_dcscmv_analysed with val == NULL then uses these values and skips
- * the per-call gather (a CSR product's cost).  Bind again after the values
- * change. */
+ * the per-call gather (a CSR product's cost).  There is room for one set: a
+ * product with values of its own puts those in their place.  Bind again
+ * after that, and after the values change. */
 SBLAS_API int sblas_csc_bind_values(int m, int n, long long nnz, const double *val, void *work,
                                     size_t work_bytes, void *stream);
 

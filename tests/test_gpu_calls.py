@@ -415,3 +415,28 @@ def test_plans_picked_for_short_and_long_rows(sblas_lib, cuda, k, m, nnz):
         assert float((y - ref).norm() / ref.norm()) <= RTOL_L2
     if nnz < 4 * m:
         assert plan.s <= 8 and batch.s <= 8
+
+
+@pytest.mark.parametrize("nnz", [5000, 300_000])
+def test_analysed_csc_product_without_values_uses_the_last_ones(sblas_lib, cuda, nnz):
+    """val = None: the values that the plan holds in row order, whether bind() or
+    a product put them there last."""
+    from hpda_sblas_pnnl_gb300 import ops
+    m, n = 4000, 3000
+    colptr, rows, cols = csc_pattern(m, n, nnz, nnz)
+    rng = np.random.default_rng(3)
+    a, b, x = rng.standard_normal(nnz), rng.standard_normal(nnz), rng.standard_normal(n)
+    cp, ri, ta, tb, tx = (torch.from_numpy(t).to(cuda) for t in (colptr, rows, a, b, x))
+    plan = ops.CscPlan(m, cp, ri)
+    y = torch.empty(m, dtype=torch.float64, device=cuda)
+    with pytest.raises(ValueError):
+        plan(None, tx, y)
+    plan.bind(ta)
+    of_a = plan(None, tx, y).clone()
+    ref = np.zeros(m)
+    np.add.at(ref, rows, a * x[cols])
+    assert rel_l2(of_a.cpu().numpy(), ref) <= RTOL_L2
+    of_b = plan(tb, tx, y).clone()
+    assert torch.equal(plan(None, tx, y), of_b) and not torch.equal(of_a, of_b)
+    plan.bind(ta)
+    assert torch.equal(plan(None, tx, y), of_a)
