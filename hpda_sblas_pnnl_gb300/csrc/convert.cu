@@ -38,16 +38,16 @@ __device__ __forceinline__ void rows_start_at(int prev, int cur, int m, long lon
         for (int r = from; r < last; ++r) rowptr[r] = (int)k;
 }
 
-// One nonzero per thread (row arrays that are not 16-byte aligned); an index
-// outside [0, m) or a decrease (unsorted input) writes nothing.
+// One nonzero per thread (row arrays that are not 16-byte aligned); an index of
+// m or more counts as row m - 1, a decrease (unsorted input) writes nothing.
 __global__ void coo_rowptr_kernel(int m, long long nnz, const int *__restrict__ row,
                                   int *__restrict__ rowptr)
 {
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k <= nnz; k += stride) {
-        const int prev = (k == 0) ? -1 : __ldg(row + k - 1);
-        const int cur = (k == nnz) ? m : __ldg(row + k);
-        if ((k < nnz && (cur < 0 || cur >= m)) || cur < prev) continue;
+        int prev = (k == 0) ? -1 : __ldg(row + k - 1);
+        if (k == nnz) prev = min(prev, m - 1);   // rowptr[m] is always written
+        const int cur = (k == nnz) ? m : min(__ldg(row + k), m - 1);
         // rows prev+1 .. cur start at k (row `cur` itself starts at k too)
         rows_start_at(prev, cur, m, k, rowptr);
     }
@@ -60,7 +60,8 @@ __global__ void coo_rowptr_kernel(int m, long long nnz, const int *__restrict__ 
 // nonzero.  19.4M nonzeros, 1M rows: 22 us and 4 us of partition -> 16 us.
 // part (may be null): the tile partition of the row pointer, for tiles of
 // `tile` nonzeros: the row of a tile's first nonzero is that nonzero's row
-// index, so no pass over the row pointer is needed.
+// index (at most m - 1, as in the row pointer: a tile never begins past the last
+// row), so no pass over the row pointer is needed.
 constexpr int COO_THREADS = 256;
 constexpr int COO_ILP = 4;
 
@@ -84,7 +85,7 @@ __global__ void __launch_bounds__(COO_THREADS) coo_rowptr_quad_kernel(
     if (part != nullptr) {
         const long long stride = (long long)gridDim.x * COO_THREADS;
         for (long long t = (long long)blockIdx.x * COO_THREADS + threadIdx.x; t <= ntiles; t += stride)
-            part[t] = t == 0 ? 0 : t == ntiles ? m : min(max(__ldg(row + t * tile), 0), m);
+            part[t] = t == 0 ? 0 : t == ntiles ? m : min(max(__ldg(row + t * tile), 0), m - 1);
     }
 #pragma unroll
     for (int i = 0; i < COO_ILP; ++i) {
@@ -102,7 +103,8 @@ __global__ void __launch_bounds__(COO_THREADS) coo_rowptr_quad_kernel(
     if (blockIdx.x == gridDim.x - 1) {
         const long long k = 4 * nq + threadIdx.x;
         if (k <= nnz) {
-            const int prev = (k == 0) ? -1 : __ldg(row + k - 1);
+            int prev = (k == 0) ? -1 : __ldg(row + k - 1);
+            if (k == nnz) prev = min(prev, m - 1);   // rowptr[m] is always written
             const int cur = (k == nnz) ? m : min(__ldg(row + k), m - 1);
             rows_start_at(prev, cur, m, k, rowptr);
         }

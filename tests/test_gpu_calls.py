@@ -440,3 +440,30 @@ def test_analysed_csc_product_without_values_uses_the_last_ones(sblas_lib, cuda,
     assert torch.equal(plan(None, tx, y), of_b) and not torch.equal(of_a, of_b)
     plan.bind(ta)
     assert torch.equal(plan(None, tx, y), of_a)
+
+
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("m,nnz,last", [(1, 5, 5), (700, 9000, 1), (700, 300_001, 100_000),
+                                        (5000, 300_000, 300_000)])
+def test_coo_rows_past_the_end_stay_inside(sblas_lib, cuda, offset, m, nnz, last):
+    """Sorted row indices of m and more (counted from one, say): taken as the
+    last row by the row pointer and by the tile partition alike, over many
+    tiles too; nothing is written behind y or the row pointer."""
+    from hpda_sblas_pnnl_gb300 import ops
+    rng = np.random.default_rng(nnz)
+    n = 300
+    rows = np.sort(rng.integers(0, m, nnz)).astype(np.int32)
+    rows[nnz - last:] = np.sort(rng.integers(m, m + 3, last))
+    col, val, x = rng.integers(0, n, nnz).astype(np.int32), rng.standard_normal(nnz), rng.standard_normal(n)
+    ref = np.zeros(m)
+    np.add.at(ref, np.minimum(rows, m - 1), val * x[col])
+    pad = torch.zeros(nnz + offset, dtype=torch.int32, device=cuda)
+    pad[offset:] = torch.from_numpy(rows).to(cuda)
+    tc, tv, tx = (torch.from_numpy(a).to(cuda) for a in (col, val, x))
+    for sigma in (0, 11, 27):
+        y = torch.full((m + 64,), -7.0, dtype=torch.float64, device=cuda)
+        rp = torch.full((m + 1 + 64,), -7, dtype=torch.int32, device=cuda)
+        ops.coomv(pad[offset:], tc, tv, tx, y[:m], rowptr_work=rp[:m + 1], sigma=sigma)
+        assert bool((y[m:] == -7.0).all()) and bool((rp[m + 1:] == -7).all())
+        assert int(rp[m]) == nnz
+        assert rel_l2(y[:m].cpu().numpy(), ref) <= RTOL_L2
