@@ -22,16 +22,18 @@
 // and positions are computed, not claimed with atomics: every run produces
 // the same output.
 //
-// Bound: the SM's store path, one request per 128-byte line that a warp's store
-// touches: three arrays in runs of T / nb = 4 entries are ~27 requests per 32
-// entries.  20M entries, 1024 digits, keys, columns and values: 234 us a pass
-// (a coalesced move of the same bytes 119 us, their HBM time 94 us).  Two
-// passes of up to 11 bits beat three of 8 all the same: 194 us each at 128
-// digits.  Equal digits by ballots rather than __match_any_sync, which takes a
+// Bound: latency.  A tile's phases (ranks, runs, keys, values, columns) wait for
+// one another, at 24 warps per SM (registers), and no unit is above 60 % of its
+// rate; the stores, one request per 128-byte line that a warp's store touches
+// (~27 per 32 entries with three arrays in runs of T / nb = 4), are one
+// contributor.  20M entries, 1024 digits, keys, columns and values, before the
+// prefetches below: 234 us a pass (a coalesced move of the same bytes 119 us,
+// their HBM time 94 us).  Two passes of up to 11 bits beat three of 8 all the
+// same: 194 us each at 128 digits.  Equal digits by ballots rather than __match_any_sync, which takes a
 // warp's distinct values one after another: 312 -> 289 us in a copy of the
 // pass; CTAs of 512 threads (twice the warp-private tables): 326 us.
-// CSC to CSR, 20M entries, 1M rows: 890 -> 523 us; one product of a CSC matrix
-// with 4.5M entries: 275 -> 155 us.
+// CSC to CSR, 20M entries, 1M rows, as a call: 890 -> 528 us; one product of a CSC
+// matrix with 4.5M entries: 275 -> 155 us.
 #pragma once
 
 #include <atomic>
@@ -571,7 +573,7 @@ __global__ void __launch_bounds__(THREADS, 3) bucket_scatter_kernel(
     // The arrays that are moved after the keys on their way to L2 from the start,
     // one prefetch per 64 bytes: a tile's phases wait for their loads one after
     // another, and holding the values in registers meanwhile spills (20M
-    // entries 594 -> 691 us).  Prefetched: 594 -> 523, 4.5M entries 142 -> 128 (one
+    // entries 594 -> 691 us of device time).  Prefetched: 594 -> 523, 4.5M entries 142 -> 128 (one
     // prefetch per 128 bytes 562 / 137; a tile of the next wave as well 547 / 133).
     constexpr int PF = 64;
     if (op.d_out)
